@@ -3,8 +3,9 @@
 // RD<T2, R, SG>::run(v) replaces v[0..R) (natural order) by its DFT
 //   X[k] = sum_n v[n] exp(SG * 2 pi i n k / R)      (SG = -1 forward, +1 inverse)
 // in natural order.  Lengths 2, 3, 4, 8 use the butterflies of fft_ct.cuh;
-// 6, 12, 16, 24 are four-step compositions R = R1 R2 whose twiddles are
-// constants computed by the compiler (Taylor series of cos and sin of the
+// 5, 7, 11, 13 pair the terms j and R - j (prime_dft); 6, 9, 10, 12, 16, 24
+// are four-step compositions R = R1 R2.  Their twiddles are constants
+// computed by the compiler (Taylor series of cos and sin of the
 // angle reduced to the first octant, exact at multiples of pi/2), so no
 // table is read.
 #pragma once
@@ -114,6 +115,34 @@ __device__ __forceinline__ void comp_dft(T2 (&v)[R1 * R2]) {
   }
 }
 
+// odd prime R: X[k], X[R-k] = a +- SG i b with a = v0 + sum_j cos(2 pi j k / R)
+// (v[j] + v[R-j]) and b = sum_j sin(2 pi j k / R) (v[j] - v[R-j]), j = 1..(R-1)/2
+template <typename T2, int R, int SG>
+__device__ __forceinline__ void prime_dft(T2 (&v)[R]) {
+  typedef typename CT<T2>::R Rt;
+  constexpr int H = (R - 1) / 2;
+  T2 s[H], d[H], x0 = v[0];
+#pragma unroll
+  for (int j = 0; j < H; ++j) {
+    s[j] = add(v[j + 1], v[R - 1 - j]);
+    d[j] = sub(v[j + 1], v[R - 1 - j]);
+    v[0] = add(v[0], s[j]);
+  }
+  sfor<1, H + 1>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    T2 a = x0, b = CT<T2>::mk(0, 0);
+    sfor<1, H + 1>([&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      constexpr Rt c = (Rt)cos2pi(j * k, R), sn = (Rt)sin2pi(j * k, R);
+      a = CT<T2>::mk(a.x + c * s[j - 1].x, a.y + c * s[j - 1].y);
+      b = CT<T2>::mk(b.x + sn * d[j - 1].x, b.y + sn * d[j - 1].y);
+    });
+    const T2 ib = mul_si(b, SG);
+    v[k] = add(a, ib);
+    v[R - k] = sub(a, ib);
+  });
+}
+
 template <typename T2, int SG>
 struct RD<T2, 1, SG> {
   static __device__ __forceinline__ void run(T2 (&)[1]) {}
@@ -137,6 +166,30 @@ struct RD<T2, 8, SG> {
 template <typename T2, int SG>
 struct RD<T2, 6, SG> {
   static __device__ __forceinline__ void run(T2 (&v)[6]) { comp_dft<T2, 2, 3, SG>(v); }
+};
+template <typename T2, int SG>
+struct RD<T2, 5, SG> {
+  static __device__ __forceinline__ void run(T2 (&v)[5]) { prime_dft<T2, 5, SG>(v); }
+};
+template <typename T2, int SG>
+struct RD<T2, 7, SG> {
+  static __device__ __forceinline__ void run(T2 (&v)[7]) { prime_dft<T2, 7, SG>(v); }
+};
+template <typename T2, int SG>
+struct RD<T2, 11, SG> {
+  static __device__ __forceinline__ void run(T2 (&v)[11]) { prime_dft<T2, 11, SG>(v); }
+};
+template <typename T2, int SG>
+struct RD<T2, 13, SG> {
+  static __device__ __forceinline__ void run(T2 (&v)[13]) { prime_dft<T2, 13, SG>(v); }
+};
+template <typename T2, int SG>
+struct RD<T2, 9, SG> {
+  static __device__ __forceinline__ void run(T2 (&v)[9]) { comp_dft<T2, 3, 3, SG>(v); }
+};
+template <typename T2, int SG>
+struct RD<T2, 10, SG> {
+  static __device__ __forceinline__ void run(T2 (&v)[10]) { comp_dft<T2, 2, 5, SG>(v); }
 };
 template <typename T2, int SG>
 struct RD<T2, 12, SG> {

@@ -12,11 +12,12 @@
 //     inverse, without the reference's temporary copy;
 //   fc_filter_r (pseudospec_hd.f90:443-467) and dlr (pseudospec_hd.f90:254-288)
 //     likewise.
-// Two kernels do the transform in shared memory: zfft2_kernel for the
+// Three kernels do the transform in shared memory: zfft2_kernel for the
 // lengths N = R1 R2 with a two-step register split (every compile-time
 // length up to 256: two shared-memory passes, results stored from
-// registers), zfft_kernel with radix passes for the others (nz 512, lengths
-// without a compile-time transform, tuned column widths).  Batches run the
+// registers), zfft_kernel with compile-time radix passes for nz 512, and
+// zfft_gen_kernel with the out-of-place passes of fft_gen.cuh for every
+// other length.  Batches run the
 // forward transforms of all their problems with one z length as one launch
 // of zfft2_group_kernel (the same body, one column block per CTA).
 #include <algorithm>
@@ -24,6 +25,7 @@
 
 #include "fft3.cuh"
 #include "fft_ct.cuh"
+#include "fft_gen.cuh"
 
 namespace {
 
@@ -45,26 +47,6 @@ struct ZArgs {
   const double* zinv2;    // nz
   const int* ell;         // nlm
   FftDesc fd;
-};
-
-template <int CTN>
-struct ZGeo {
-  typedef ct::Geo<CTN, 0, false> type;
-  static __device__ __forceinline__ type make(int LB, int) { return type{LB, 1, LB}; }
-};
-template <>
-struct ZGeo<0> {
-  typedef FftGeom type;
-  static __device__ __forceinline__ type make(int LB, int n) {
-    FftGeom g;
-    g.n = n;
-    g.batch = LB;
-    g.bs = 1;
-    g.es = LB;
-    g.pad = 0;
-    g.jfast = false;
-    return g;
-  }
 };
 
 // 16-byte global -> shared copy that lands asynchronously; src_bytes 0
@@ -157,14 +139,9 @@ __global__ void __launch_bounds__(ZTHREADS) zfft_kernel(ZArgs a) {
     __syncthreads();
   }
 
-  const auto g = ZGeo<CTN>::make(LB, nz);
-  if (MODE == Z_INV) {
-    if constexpr (CTN > 0) ct::dit<double2, CTN, CTN>(sm, g, a.fd.twp, +1);
-    else fft_dit(sm, a.fd, g, +1);
-  } else {
-    if constexpr (CTN > 0) ct::dif<double2, CTN, CTN>(sm, g, a.fd.twp, -1);
-    else fft_dif(sm, a.fd, g, -1);
-  }
+  const ct::Geo<CTN, 0, false> g{LB, 1, LB};
+  if (MODE == Z_INV) ct::dit<double2, CTN, CTN>(sm, g, a.fd.twp, +1);
+  else ct::dif<double2, CTN, CTN>(sm, g, a.fd.twp, -1);
 
   if (MODE == Z_DERIV || MODE == Z_FILTER || MODE == Z_DLR) {
     // spectral multiply in place (frequency k sits at row rev[k]), then back
@@ -177,8 +154,7 @@ __global__ void __launch_bounds__(ZTHREADS) zfft_kernel(ZArgs a) {
       sm[o] = v;
     }
     __syncthreads();
-    if constexpr (CTN > 0) ct::dit<double2, CTN, CTN>(sm, g, a.fd.twp, +1);
-    else fft_dit(sm, a.fd, g, +1);
+    ct::dit<double2, CTN, CTN>(sm, g, a.fd.twp, +1);
   }
 
   for (int idx = tid; idx < nz * LB; idx += ZTHREADS) {
@@ -326,6 +302,94 @@ __global__ void __launch_bounds__(Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::THR
   zfft2_body<MODE, R1, R2, IO>(jobs[lo], (int)blockIdx.x - __ldg(prefix + lo));
 }
 
+// Lengths without a compile-time transform: the slab in natural order, the
+// out-of-place passes of fft_gen.cuh between two buffers (a third keeps the
+// D_l input), then one store.  Bound by the latency of the passes where a
+// call has few columns and by shared memory where it has many.  Derivative of
+// 528 columns at nz 58 (2 29) and 33 (3 11): 7.1 and 6.3 us, against 221 and
+// 42 us with one thread per butterfly in place and 32 columns per CTA; nz 90,
+// 14706 columns, plain: 19-27 against 52-59 us.
+template <int MODE, int IO>
+__global__ void __launch_bounds__(ZTHREADS, 2) zfft_gen_kernel(ZArgs a, int lg) {
+  extern __shared__ double2 sm[];
+  const int LB = 1 << lg, nz = a.nz, nlm = a.nlm, lm0 = blockIdx.x << lg, tid = threadIdx.x;
+  const bool cont = MODE != Z_INV && a.C > 0;
+  const int nload = cont ? a.N : nz, total = nz << lg;
+  double2* orig = sm + 2 * total;  // D_l keeps the input column for the l(l+1)/r^2 term
+  for (int idx = tid; idx < nload << lg; idx += ZTHREADS) {
+    const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
+    zload<IO>(a, sm + idx, (size_t)r * nlm + lm, lm < nlm);
+  }
+  if (MODE == Z_DLR)
+    for (int idx = tid; idx < total; idx += ZTHREADS) {
+      const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
+      zload<IO>(a, orig + idx, (size_t)r * nlm + lm, lm < nlm);
+    }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  if (cont) {  // as in zfft_kernel
+    for (int idx = tid; idx < a.C << lg; idx += ZTHREADS) {
+      const int ii = idx >> lg, c = idx & (LB - 1);
+      sm[((a.N + ii) << lg) + c] = fc_cont_elem(a.dir, a.C, a.d, a.N, ii, sm + c, LB);
+    }
+    __syncthreads();
+  }
+  constexpr int SG = MODE == Z_INV ? 1 : -1;  // first transform's sign
+  double2* x = fg::run<SG>(sm, sm + total, nz, a.fd.gf, 0, a.fd.ng, lg, a.fd.tw);
+  if constexpr (MODE == Z_DERIV || MODE == Z_FILTER || MODE == Z_DLR) {
+    for (int idx = tid; idx < total; idx += ZTHREADS) {
+      const int k = idx >> lg;
+      const double2 v = div_nz(x[idx], nz);
+      x[idx] = MODE == Z_FILTER ? cscale(v, a.filt[k]) : cmul(a.kfac[k], v);
+    }
+    __syncthreads();
+    x = fg::run<1>(x, x == sm ? sm + total : sm, nz, a.fd.gf, 0, a.fd.ng, lg, a.fd.tw);
+  }
+  for (int idx = tid; idx < total; idx += ZTHREADS) {
+    const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
+    if (lm >= nlm) continue;
+    double2 v = MODE == Z_FWD ? div_nz(x[idx], nz) : x[idx];
+    if (MODE == Z_DLR) {
+      // b = b + z^-2 * (-l(l+1) a)   (laplang, multr(-2), saxpby_c)
+      const double lf = -(double)(a.ell[lm] * (a.ell[lm] + 1));
+      const double2 o = orig[idx];
+      const double zi = a.zinv2[r];
+      v.x = v.x + zi * (lf * o.x);
+      v.y = v.y + zi * (lf * o.y);
+    }
+    zstore<IO>(a, (size_t)r * nlm + lm, v);
+  }
+}
+
+// Columns per CTA of zfft_gen_kernel where the plan sets none: the default
+// slab (32 KB), halved down to 4 columns while the grid has fewer than two
+// CTAs per SM (a 528-column derivative at nz 58 then has 132 CTAs, not 17).
+int zgen_lb(int nz, int nlm) {
+  int lb = 64;
+  while (lb > 1 && lb * nz > ZMAXCOL / 2) lb >>= 1;
+  while (lb > 4 && (nlm + lb - 1) / lb < 2 * 148) lb >>= 1;
+  return lb;
+}
+
+template <int MODE, int IO>
+int launch_gen(const ZArgs& a, cudaStream_t st) {
+  static DeviceOnce once;
+  if (!once.run([] {
+        return cudaFuncSetAttribute(zfft_gen_kernel<MODE, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    200 * 1024) == cudaSuccess &&
+               cudaFuncSetAttribute(zfft_gen_kernel<MODE, IO>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    100) == cudaSuccess;
+      }))
+    return SPH_ECUDA;
+  int lg = 0;
+  while ((1 << lg) < a.LB) ++lg;
+  const size_t smem = ((size_t)a.nz << lg) * sizeof(double2) * (MODE == Z_DLR ? 3 : 2);
+  zfft_gen_kernel<MODE, IO><<<(a.nlm + a.LB - 1) / a.LB, ZTHREADS, smem, st>>>(a, lg);
+  SPH_LAUNCH_OK();
+  return SPH_OK;
+}
+
 template <int MODE, int CTN, int IO>
 int launch_ct(const ZArgs& a, int nblocks, size_t smem, cudaStream_t st) {
   static DeviceOnce once;
@@ -371,6 +435,16 @@ bool zsplit_length(int nz) {
   return false;
 }
 
+bool ct_length(int nz) {
+  switch (nz) {
+#define CASE(n) case n:
+    Z_SIZES(CASE)
+#undef CASE
+    return true;
+  }
+  return false;
+}
+
 template <int MODE, int IO>
 int launch_mode(const ZArgs& a, int nblocks, size_t smem, cudaStream_t st) {
   switch (a.nz) {
@@ -378,7 +452,7 @@ int launch_mode(const ZArgs& a, int nblocks, size_t smem, cudaStream_t st) {
   case n: return launch_ct<MODE, n, IO>(a, nblocks, smem, st);
     Z_SIZES(CASE)
 #undef CASE
-    default: return launch_ct<MODE, 0, IO>(a, nblocks, smem, st);
+    default: return launch_gen<MODE, IO>(a, st);
   }
 }
 
@@ -434,6 +508,7 @@ int make_zargs(const sph_plan* p, int mode, const void* in, void* out, int order
   while (LB > 1 && LB * p->nz > ZMAXCOL / 2) LB >>= 1;
   // a tuned width, except for the lengths with the two-step split, whose
   // kernel is compiled for the default width
+  if (!ct_length(p->nz)) LB = zgen_lb(p->nz, p->nlmv);
   if (p->tile_lb && !zsplit_length(p->nz)) LB = p->tile_lb;
   if (LB * p->nz > ZMAXCOL) return SPH_EINVAL;
   a.LB = LB;
@@ -627,10 +702,12 @@ extern "C" int sph_derivr_noalloc(const double* a, double* b, int nlm, int nz, i
         r /= q;
       }
   }
+  if (!fft_gen_plan(nz, fd)) return SPH_EINVAL;
   int LB = 64;
   // the column blocks of the plan path (so that both run the same kernel)
   while (LB > 1 && LB * nz > ZMAXCOL / 2) LB >>= 1;
   if (LB * nz > ZMAXCOL) return SPH_EINVAL;
+  if (!ct_length(nz)) LB = zgen_lb(nz, nlm);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return SPH_ECUDA;
   std::lock_guard<std::mutex> lock(na_mutex);

@@ -13,6 +13,7 @@
 #include <thread>
 
 #include "fft_ct.cuh"
+#include "fft_gen.cuh"
 #include "sph_internal.cuh"
 
 typedef long double ld;
@@ -255,7 +256,8 @@ extern "C" int sph_plan_create(sph_plan** out, int lmax, int nlat, int nphi, int
   p->precision = precision;
   p->rint = rint;
   p->rext = rext;
-  if (fft_factor(nz, p->fz) || fft_factor(nphi, p->fphi)) {
+  if (fft_factor(nz, p->fz) || fft_factor(nphi, p->fphi) || !fft_gen_plan(nz, p->fz) ||
+      !fft_gen_plan(nphi, p->fphi)) {
     delete p;
     return SPH_EINVAL;
   }

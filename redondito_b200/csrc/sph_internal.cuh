@@ -21,6 +21,15 @@ struct FftPass {
   int R, Ns;
 };
 
+// One pass of the out-of-place engine (fft_gen.cuh): radix R, span s (the
+// product of the radices before it), mul = ceil(2^32 / s) for t / s.
+struct GenPass {
+  int R, s;
+  unsigned mul;
+};
+#define SPH_GEN_PASSES 8
+#define SPH_GEN_RADIX 13  // largest radix done as one register butterfly
+
 // A length-n complex FFT in shared memory.  tw[e] = exp(-2 pi i e / n);
 // rev[k] = position of frequency k after the decimation-in-frequency passes.
 struct FftDesc {
@@ -31,6 +40,10 @@ struct FftDesc {
   const int* rev;
   const double2* twp;   // per-pass table [pass][j][r-1] = W_L^{j r} (compile-time lengths)
   const float2* twpf;
+  // out-of-place passes (fft_gen.cuh): register radices first, larger primes
+  // after them (gf), and the reverse (gl: register radices last)
+  int ng;
+  GenPass gf[SPH_GEN_PASSES], gl[SPH_GEN_PASSES];
 };
 
 // Legendre GEMM work tile: one (m, row block) pair.
