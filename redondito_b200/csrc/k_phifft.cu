@@ -12,12 +12,14 @@
 //   G[m][1][k][i] = W_i (F_m(i) - F_m(mirror))   (odd part)
 // with W_i = w_i 2 pi / nphi; the inverse kernel reads the same layout
 // (synthesised even/odd sums) and writes both rings of the grid.
-// Lengths 2^a 3^b use the compile-time FFT of fft_ct.cuh; others the
-// runtime engine of fft_engine.cuh.
+// Lengths 3 2^a use compile-time FFTs (fft3.cuh, fft_ct.cuh); others the
+// out-of-place passes of fft_gen.cuh, or, past the length whose two buffers
+// fit shared memory, the in-place engine of fft_engine.cuh.
 #include <algorithm>
 
 #include "fft3.cuh"
 #include "fft_ct.cuh"
+#include "fft_gen.cuh"
 #include "tc05.cuh"
 #include "tma.cuh"
 #include "cluster.cuh"
@@ -167,7 +169,175 @@ __global__ void __launch_bounds__(PTHREADS, 2) phi_inv_ct(PhiArgs a) {
 }
 
 // ---------------------------------------------------------------- other lengths
-template <int CTN>
+// NB = 1 << lg ring pairs per CTA, the out-of-place passes of fft_gen.cuh.
+// The forward transform's first pass takes its butterflies straight from the
+// grid rows (2 R loads in flight per thread) and the inverse's last pass
+// writes its outputs straight to them, so only the passes between move the
+// tile through shared memory; a length whose factors are all above
+// SPH_GEN_RADIX loads or stores the tile in a pass of its own.  The last
+// tile may hold fewer ring pairs than NB.  260 x 520 (13 8 5), 90 planes, per
+// field: forward 94 us, inverse 69 us; one thread per butterfly in place with
+// 2 ring pairs per CTA (16-byte runs of a grid row) took 645 us each.
+template <int R>
+__device__ __noinline__ void phi_gen_first(const double* ring, const double* mirror, int nlat, int np, double2* dst,
+                                           int n, GenPass g, int lg, const double2* __restrict__ tw) {
+  const int nt = n / R;
+  for (int it = threadIdx.x; it < nt << lg; it += blockDim.x) {
+    const int b = it & ((1 << lg) - 1), t = it >> lg;
+    double2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const size_t j = (size_t)(t + r * nt) * nlat;
+      v[r] = b < np ? make_double2(__ldg(ring + j + b), __ldg(mirror + j - b)) : make_double2(0.0, 0.0);
+    }
+    ct::RD<double2, R, -1>::run(v);
+    fg::put<R, -1>(dst, v, t, b, g, lg, tw);
+  }
+}
+
+template <int R>
+__device__ __noinline__ void phi_gen_last(const double2* src, double* ring, double* mirror, int nlat, int np, int n,
+                                          int lg) {
+  const int nt = n / R;
+  for (int it = threadIdx.x; it < nt << lg; it += blockDim.x) {
+    const int b = it & ((1 << lg) - 1), t = it >> lg;
+    if (b >= np) continue;
+    double2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = src[((t + r * nt) << lg) + b];
+    ct::RD<double2, R, 1>::run(v);
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const size_t j = (size_t)(t + k * nt) * nlat;
+      ring[j + b] = v[k].x;
+      mirror[j - b] = v[k].y;
+    }
+  }
+}
+
+constexpr int GENT = 320;  // most threads of the general-length kernels
+
+__global__ void __launch_bounds__(GENT, 2) phi_fwd_gen(PhiArgs a, int lg) {
+  extern __shared__ double2 sm[];
+  const int NB = 1 << lg, n = a.nphi, nlat = a.nlat, p0 = blockIdx.x << lg, tid = threadIdx.x;
+  const int k = a.kzl ? __ldg(a.kzl + blockIdx.y) : blockIdx.y, f = blockIdx.z;
+  const int np = min(NB, a.nlat2 - p0);
+  const double* plane = a.gin[f] + (size_t)k * n * nlat;
+  const double *ring = plane + p0, *mirror = plane + nlat - 1 - p0;
+  double2* x = sm;
+  int ip = 0;
+  switch (a.fd.ng ? a.fd.gf[0].R : 0) {
+#define CASE(r) \
+  case r: phi_gen_first<r>(ring, mirror, nlat, np, x, n, a.fd.gf[0], lg, a.fd.tw); ip = 1; break;
+    SPH_GEN_RADICES(CASE)
+#undef CASE
+    default:
+      for (int it = tid; it < n << lg; it += blockDim.x) {
+        const int b = it & (NB - 1);
+        const size_t j = (size_t)(it >> lg) * nlat;
+        x[it] = b < np ? make_double2(__ldg(ring + j + b), __ldg(mirror + j - b)) : make_double2(0.0, 0.0);
+      }
+  }
+  __syncthreads();
+  x = fg::run<-1>(x, sm + (n << lg), n, a.fd.gf, ip, a.fd.ng, lg, a.fd.tw);
+  // both parities of one (m, pair) from Z(m), Z(-m), as phi_fwd_ct
+  double2* G = a.G + (size_t)f * a.Gfield + (size_t)k * a.ldn + p0;
+  const size_t pstride = (size_t)a.nz * a.ldn;
+  for (int it = tid; it < (a.lmax + 1) << lg; it += blockDim.x) {
+    const int b = it & (NB - 1), m = it >> lg;
+    if (b >= np) continue;
+    const double2 Z = x[it], Zc = x[((m == 0 ? 0 : n - m) << lg) + b];
+    const double2 Fi = make_double2(0.5 * (Z.x + Zc.x), 0.5 * (Z.y - Zc.y));
+    const double2 Fm = make_double2(0.5 * (Z.y + Zc.y), -0.5 * (Z.x - Zc.x));
+    const double W = __ldg(a.wfold + p0 + b);
+    double2* o = G + (size_t)m * 2 * pstride + b;
+    o[0] = cscale(cadd(Fi, Fm), W);
+    o[pstride] = cscale(csub(Fi, Fm), W);
+  }
+}
+
+__global__ void __launch_bounds__(GENT, 2) phi_inv_gen(PhiArgs a, int lg) {
+  extern __shared__ double2 sm[];
+  const int NB = 1 << lg, n = a.nphi, nlat = a.nlat, p0 = blockIdx.x << lg, tid = threadIdx.x;
+  const int k = a.kzl ? __ldg(a.kzl + blockIdx.y) : blockIdx.y, f = blockIdx.z;
+  const int np = min(NB, a.nlat2 - p0), M = a.lmax + 1;
+  // Z(m) of each ring pair (ring + i mirror): 2 lmax + 1 frequencies, zero between
+  const double2* G = a.Gc + (size_t)f * a.Gfield + (size_t)k * a.ldn + p0;
+  const size_t pstride = (size_t)a.nz * a.ldn;
+  for (int it = (M << lg) + tid; it < (n - M + 1) << lg; it += blockDim.x) sm[it] = make_double2(0.0, 0.0);
+#pragma unroll 4
+  for (int it = tid; it < M << lg; it += blockDim.x) {
+    const int b = it & (NB - 1), m = it >> lg;
+    const double2* c = G + (size_t)m * 2 * pstride + b;
+    const double2 zero = make_double2(0.0, 0.0);
+    const double2 se = b < np ? __ldg(c) : zero, so = b < np ? __ldg(c + pstride) : zero;
+    const double2 Fi = cadd(se, so), Fm = csub(se, so);
+    if (m == 0) {
+      sm[b] = make_double2(Fi.x, Fm.x);
+    } else {
+      sm[it] = make_double2(Fi.x - Fm.y, Fi.y + Fm.x);
+      sm[((n - m) << lg) + b] = make_double2(Fi.x + Fm.y, -Fi.y + Fm.x);
+    }
+  }
+  __syncthreads();
+  const int ng = a.fd.ng, rl = ng ? a.fd.gl[ng - 1].R : 0;
+  const bool direct = rl >= 2 && rl <= SPH_GEN_RADIX;
+  const double2* x = fg::run<1>(sm, sm + (n << lg), n, a.fd.gl, 0, direct ? ng - 1 : ng, lg, a.fd.tw);
+  double* plane = a.gout[f] + (size_t)k * n * nlat;
+  double *ring = plane + p0, *mirror = plane + nlat - 1 - p0;
+  switch (direct ? rl : 0) {
+#define CASE(r) \
+  case r: phi_gen_last<r>(x, ring, mirror, nlat, np, n, lg); break;
+    SPH_GEN_RADICES(CASE)
+#undef CASE
+    default:
+      for (int it = tid; it < n << lg; it += blockDim.x) {
+        const int b = it & (NB - 1);
+        if (b >= np) continue;
+        const size_t j = (size_t)(it >> lg) * nlat;
+        ring[j + b] = x[it].x;
+        mirror[j - b] = x[it].y;
+      }
+  }
+}
+
+// Ring pairs and threads per CTA of the general-length kernels: the tuned
+// ring pairs, else the most of 8, 4, 2 and 1 whose two buffers let two CTAs
+// share an SM (longer runs of a grid row against more loads in flight); then
+// the threads that leave the fewest lanes idle over the passes.  False: even
+// one pair's buffers exceed shared memory.
+bool phi_gen_geometry(const sph_plan* p, int* lg, int* threads, size_t* smem) {
+  const size_t pair = 2 * (size_t)p->nphi * sizeof(double2);
+  int l = 0;
+  if (p->tile_np) {
+    while ((1 << l) < p->tile_np) ++l;
+    while (l > 0 && (pair << l) > 200 * 1024) --l;
+  } else {
+    l = 3;
+    while (l > 0 && (pair << l) > 110 * 1024) --l;
+  }
+  if ((pair << l) > 200 * 1024) return false;
+  long long least = 0;
+  *threads = 0;
+  for (int t = 128; t <= GENT; t += 32) {
+    long long slots = 0;
+    for (int i = 0; i < p->fphi.ng; ++i) {
+      const GenPass& g = p->fphi.gf[i];
+      const bool big = g.R > SPH_GEN_RADIX;
+      const long long items = ((long long)(p->nphi / g.R) * (big ? (g.R + 1) / 2 : 1)) << l;
+      slots += (items + t - 1) / t * t * (big ? 2 : 1) * g.R;
+    }
+    if (!*threads || slots <= least) {
+      *threads = t;
+      least = slots;
+    }
+  }
+  *lg = l;
+  *smem = pair << l;
+  return true;
+}
+
+// the in-place engine: lengths whose two buffers do not fit shared memory
 __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd_kernel(PhiArgs a) {
   extern __shared__ double2 sm[];
   const int NP = a.NP, nphi = a.nphi, nlat = a.nlat, nlat2 = a.nlat2;
@@ -205,7 +375,6 @@ __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd_kernel(PhiArgs a) {
   }
 }
 
-template <int CTN>
 __global__ void __launch_bounds__(PTHREADS, 2) phi_inv_kernel(PhiArgs a) {
   extern __shared__ double2 sm[];
   const int NP = a.NP, nphi = a.nphi, nlat = a.nlat, nlat2 = a.nlat2;
@@ -740,7 +909,7 @@ int launch_fwd_n(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
       case 1: return run(phi_fwd_ct<N, 1>, a, grid, smem, st);
     }
   }
-  return run(phi_fwd_kernel<0>, a, grid, smem, st);
+  return SPH_EINVAL;
 }
 
 template <int N>
@@ -753,7 +922,7 @@ int launch_inv_n(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
       case 1: return run(phi_inv_ct<N, 1>, a, grid, smem, st);
     }
   }
-  return run(phi_inv_kernel<0>, a, grid, smem, st);
+  return SPH_EINVAL;
 }
 
 #define PHI_SIZES(X) X(12) X(24) X(48) X(96) X(192) X(384) X(768) X(1536) X(3072) X(6144)
@@ -802,8 +971,16 @@ int launch_phi_fwd(const sph_plan* p, const double* const* grids, int nfields, c
   case n: return launch_fwd_n<n>(a, grid, smem, st);
     PHI_SIZES(CASE)
 #undef CASE
-    default: return launch_fwd_n<0>(a, grid, smem, st);
+    default: break;
   }
+  int lg = 0, threads = 0;
+  size_t gsmem = 0;
+  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run(phi_fwd_kernel, a, grid, smem, st);
+  if (!smem_attr(phi_fwd_gen)) return SPH_ECUDA;
+  grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
+  phi_fwd_gen<<<grid, threads, gsmem, st>>>(a, lg);
+  SPH_LAUNCH_OK();
+  return SPH_OK;
 }
 
 int launch_phi_inv(const sph_plan* p, double* const* grids, int nfields, cudaStream_t st) {
@@ -829,6 +1006,14 @@ int launch_phi_inv(const sph_plan* p, double* const* grids, int nfields, cudaStr
   case n: return launch_inv_n<n>(a, grid, smem, st);
     PHI_SIZES(CASE)
 #undef CASE
-    default: return launch_inv_n<0>(a, grid, smem, st);
+    default: break;
   }
+  int lg = 0, threads = 0;
+  size_t gsmem = 0;
+  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run(phi_inv_kernel, a, grid, smem, st);
+  if (!smem_attr(phi_inv_gen)) return SPH_ECUDA;
+  grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
+  phi_inv_gen<<<grid, threads, gsmem, st>>>(a, lg);
+  SPH_LAUNCH_OK();
+  return SPH_OK;
 }
