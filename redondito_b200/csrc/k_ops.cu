@@ -129,42 +129,99 @@ __global__ void bc_walls_kernel(double2* tor, const double* __restrict__ neu, in
 }
 
 // invDl (boundary_mod.f90:244-292): W(1:N) = M_l phi(3:N-2) for all m of one
-// l, the reference's DGEMM with two columns (re, im) per mode.  CTA: one l and
-// up to 32 m; phi rows staged in shared memory, M_l streamed from L2.  The
-// arrays are the caller's lm columns [lm0, lm0 + nlm); modes outside are
-// skipped.
-constexpr int IDL_M = 32;
-__global__ void __launch_bounds__(256) invdl_kernel(const double2* __restrict__ phi, double2* __restrict__ w,
-                                                    const double* __restrict__ binv,
-                                                    const int* __restrict__ mbase, int lm0, int nlm, int N) {
-  extern __shared__ double2 Ph[];  // [(N-4)][IDL_M]
-  const int l = blockIdx.x + 1;
+// l, the reference's DGEMM with two columns (re, im) per mode, on the FP64
+// tensor cores (mma.m8n8k4): the scalar form took one load of M_l per two
+// FMAs and was bound by its load pipe.  CTA: one l and up to 32 m, whose phi
+// rows are staged in shared memory (K-major, 68 doubles a row: conflict-free
+// B fragments); a warp takes 16 rows of M_l, its A fragments straight from
+// L2, loaded 16 columns ahead, each used for up to 8 column tiles.  What is
+// left is bound by the 16-byte gathers and scatters of one l's modes.  lmax
+// 255: 191 -> 74 us at nz 96, 312 -> 104 us at nz 128 (16 modes per CTA, or
+// one warp per 16 rows instead of 8 warps: 79 us).  The continuation rows of
+// W and its l = 0 column are zero.  The arrays are the caller's lm columns
+// [lm0, lm0 + nlm); modes outside are skipped.
+constexpr int IDL_M = 32, IDL_NT = IDL_M / 4, IDL_LD = 2 * IDL_M + 4;
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+__global__ void __launch_bounds__(256, 2) invdl_kernel(const double2* __restrict__ phi, double2* __restrict__ w,
+                                                       const double* __restrict__ binv,
+                                                       const int* __restrict__ mbase, int lm0, int nlm, int N,
+                                                       int nz) {
+  extern __shared__ double Ph[];  // [K rounded up to 16][IDL_LD]
+  const int l = gridDim.x - blockIdx.x;  // the l with most modes first
   const int m0 = blockIdx.y * IDL_M;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const double2 zero = make_double2(0.0, 0.0);
+  if (l == 1 && m0 == 0 && lm0 == 0)  // l = 0
+    for (int k = tid; k < nz; k += 256) w[(size_t)k * nlm] = zero;
   if (m0 > l) return;
   const int nm = min(IDL_M, l + 1 - m0);
-  const int K = N - 4;
-  for (int idx = threadIdx.x; idx < K * IDL_M; idx += blockDim.x) {
-    int j = idx / IDL_M, mm = idx - j * IDL_M;
-    double2 v = make_double2(0.0, 0.0);
-    if (mm < nm) {
-      const int lm = mbase[m0 + mm] + (l - m0 - mm) - lm0;  // column of the caller's slab
-      if (lm >= 0 && lm < nlm) v = phi[(size_t)(j + 2) * nlm + lm];
-    }
-    Ph[idx] = v;
-  }
+  const int K = N - 4, KP = (K + 15) & ~15;
+  // column of mode m0 + mm in the caller's slab, -1 outside it
+  auto col = [&](int mm) {
+    const int lm = mm < nm ? __ldg(mbase + m0 + mm) + (l - m0 - mm) - lm0 : -1;
+    return lm < nlm ? lm : -1;
+  };
+  const int cm = tid % IDL_M, clm = col(cm);
+#pragma unroll 4
+  for (int j = tid / IDL_M; j < KP; j += 256 / IDL_M)
+    *reinterpret_cast<double2*>(Ph + j * IDL_LD + 2 * cm) =
+        (clm >= 0 && j < K) ? __ldg(phi + (size_t)(j + 2) * nlm + clm) : zero;
+  if (clm >= 0)
+    for (int k = N + tid / IDL_M; k < nz; k += 256 / IDL_M) w[(size_t)k * nlm + clm] = zero;
   __syncthreads();
   const double* M = binv + (size_t)(l - 1) * N * K;
-  for (int idx = threadIdx.x; idx < N * nm; idx += blockDim.x) {
-    int i = idx % N, mm = idx / N;
-    double sr = 0.0, si = 0.0;
-    for (int j = 0; j < K; ++j) {
-      double c = __ldg(M + i + (size_t)N * j);
-      double2 v = Ph[j * IDL_M + mm];
-      sr += c * v.x;
-      si += c * v.y;
+  for (int i0 = 16 * warp; i0 < N; i0 += 128) {
+    double acc[2][IDL_NT][2], a0[8], a1[8];
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < IDL_NT; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
+    // the A fragments of 16 columns from k0: rows i0 + 8 x + g, columns k0 + 4 q + t
+    auto load = [&](double (&a)[8], int k0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const int i = i0 + 8 * x + g, j = k0 + 4 * q + t;
+          a[2 * q + x] = (i < N && j < K) ? __ldg(M + i + (size_t)N * j) : 0.0;
+        }
+    };
+    auto mma = [&](const double (&a)[8], int k0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double* B = Ph + (k0 + 4 * q + t) * IDL_LD + g;
+#pragma unroll
+        for (int y = 0; y < IDL_NT; ++y)
+          if (4 * y < nm) {
+            const double b = B[8 * y];
+            dmma884(acc[0][y], a[2 * q], b);
+            dmma884(acc[1][y], a[2 * q + 1], b);
+          }
+      }
+    };
+    load(a0, 0);
+    for (int k0 = 0; k0 < KP; k0 += 32) {
+      if (k0 + 16 < KP) load(a1, k0 + 16);
+      mma(a0, k0);
+      if (k0 + 16 < KP) {
+        if (k0 + 32 < KP) load(a0, k0 + 32);
+        mma(a1, k0 + 16);
+      }
     }
-    const int lm = mbase[m0 + mm] + (l - m0 - mm) - lm0;
-    if (lm >= 0 && lm < nlm) w[(size_t)i * nlm + lm] = make_double2(sr, si);
+#pragma unroll
+    for (int y = 0; y < IDL_NT; ++y) {
+      const int lm = col(4 * y + t);
+      if (lm < 0) continue;
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const int i = i0 + 8 * x + g;
+        if (i < N) w[(size_t)i * nlm + lm] = make_double2(acc[x][y][0], acc[x][y][1]);
+      }
+    }
   }
 }
 
@@ -324,19 +381,21 @@ int launch_reconstruct(const sph_plan* p, double2* f, int boun, int ord, const d
 }
 
 int launch_invDl(const sph_plan* p, const double2* phi, double2* w, cudaStream_t st) {
-  SPH_CUDA_OK(cudaMemsetAsync(w, 0, spec_view(p) * sizeof(double2), st));
-  if (p->lmax < 1) return SPH_OK;
-  size_t smem = (size_t)(p->N - 4) * IDL_M * sizeof(double2);
-  if (smem > 200 * 1024) return SPH_EINVAL;
+  if (p->lmax < 1) {
+    SPH_CUDA_OK(cudaMemsetAsync(w, 0, spec_view(p) * sizeof(double2), st));
+    return SPH_OK;
+  }
+  if ((size_t)(p->N - 4) * 32 * sizeof(double2) > 200 * 1024) return SPH_EINVAL;
+  const size_t smem = (size_t)((p->N - 4 + 15) & ~15) * IDL_LD * sizeof(double);
   static DeviceOnce once;
   if (!once.run([] {
-        return cudaFuncSetAttribute(invdl_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
+        return cudaFuncSetAttribute(invdl_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) ==
                cudaSuccess;
       }))
     return SPH_ECUDA;
   dim3 grid(p->lmax, (p->lmax + 1 + IDL_M - 1) / IDL_M);
   TimedLaunch tl(p, T_OPS, st);
-  invdl_kernel<<<grid, 256, smem, st>>>(phi, w, p->binv, p->d_mbase, p->lm0, p->nlmv, p->N);
+  invdl_kernel<<<grid, 256, smem, st>>>(phi, w, p->binv, p->d_mbase, p->lm0, p->nlmv, p->N, p->nz);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
