@@ -212,12 +212,10 @@ struct RD<T2, 24, SG> {
 // barrier), thread h = k1 < R1: the R2-point DFT over n2 of the slots R2 h ..
 // R2 h + R2 - 1, which is X[h + R1 k2] in v[k2].  Two shared-memory passes
 // instead of one per radix pass, and the results leave from registers.
+// dft2_put1 is step 1 on values already in registers (h < R2).
 template <int R1, int R2, int SG>
-__device__ __forceinline__ void dft2_step1(double2* col, int stride, int h, const double2* __restrict__ tw) {
-  if (h >= R2) return;
-  double2 v[R1];
-#pragma unroll
-  for (int n1 = 0; n1 < R1; ++n1) v[n1] = col[(h + R2 * n1) * stride];
+__device__ __forceinline__ void dft2_put1(double2 (&v)[R1], double2* col, int stride, int h,
+                                          const double2* __restrict__ tw) {
   RD<double2, R1, SG>::run(v);
   col[h * stride] = v[0];
 #pragma unroll
@@ -228,11 +226,46 @@ __device__ __forceinline__ void dft2_step1(double2* col, int stride, int h, cons
   }
 }
 template <int R1, int R2, int SG>
+__device__ __forceinline__ void dft2_step1(double2* col, int stride, int h, const double2* __restrict__ tw) {
+  if (h >= R2) return;
+  double2 v[R1];
+#pragma unroll
+  for (int n1 = 0; n1 < R1; ++n1) v[n1] = col[(h + R2 * n1) * stride];
+  dft2_put1<R1, R2, SG>(v, col, stride, h, tw);
+}
+template <int R1, int R2, int SG>
 __device__ __forceinline__ void dft2_step2(const double2* col, int stride, int h, double2 (&v)[R2]) {
   if (h >= R1) return;
 #pragma unroll
   for (int n2 = 0; n2 < R2; ++n2) v[n2] = col[(n2 + R2 * h) * stride];
   RD<double2, R2, SG>::run(v);
+}
+// A transform back (sign SG) of a spectrum that dft2_step2 left in registers,
+// v[k2] = X[h + R1 k2]: n = a + R2 b.  Step 1, thread h = k1 < R1: the
+// R2-point DFT over k2 where the values are, times W_N^(SG a h), into the
+// thread's own R2 slots a + R2 h (the ones its step 2 read, so no barrier in
+// between).  Step 2 (after a barrier), thread h = a < R2: the R1-point DFT
+// over k1 of the slots h + R2 k1, the elements h + R2 b in v[b].  One
+// shared-memory exchange between the forward step 2 and the result.
+template <int R1, int R2, int SG>
+__device__ __forceinline__ void dft2_back1(double2 (&v)[R2], double2* col, int stride, int h,
+                                           const double2* __restrict__ tw) {
+  if (h >= R1) return;
+  RD<double2, R2, SG>::run(v);
+  col[R2 * h * stride] = v[0];
+#pragma unroll
+  for (int a = 1; a < R2; ++a) {
+    double2 w = __ldg(tw + h * a);
+    if (SG > 0) w.y = -w.y;
+    col[(a + R2 * h) * stride] = mul(v[a], w);
+  }
+}
+template <int R1, int R2, int SG>
+__device__ __forceinline__ void dft2_back2(const double2* col, int stride, int h, double2 (&v)[R1]) {
+  if (h >= R2) return;
+#pragma unroll
+  for (int k1 = 0; k1 < R1; ++k1) v[k1] = col[(h + R2 * k1) * stride];
+  RD<double2, R1, SG>::run(v);
 }
 // the first factor of the two-step split of the radial lengths with a
 // compile-time transform (0: radix passes)

@@ -1450,23 +1450,19 @@ __global__ void __launch_bounds__(ZT_THREADS, (DER && NZ >= 256) ? 2 : 3) zinv_t
     __syncthreads();
     double2 v[R2];
     if (h < TPC) ct::dft2_step2<R1, R2, -1>(col, ZT_PITCH, h, v);
-    __syncthreads();
     if (h < R1) {
 #pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) {
-        const int k = h + R1 * k2;
-        col[k * ZT_PITCH] = cmul(a.kfac[k], div_nz(v[k2], NZ));
-      }
+      for (int k2 = 0; k2 < R2; ++k2) v[k2] = cmul(a.kfac[h + R1 * k2], div_nz(v[k2], NZ));
     }
+    if (h < TPC) ct::dft2_back1<R1, R2, 1>(v, col, ZT_PITCH, h, a.tw);
     __syncthreads();
-    if (h < TPC) ct::dft2_step1<R1, R2, 1>(col, ZT_PITCH, h, a.tw);
-    __syncthreads();
-    if (h < TPC) ct::dft2_step2<R1, R2, 1>(col, ZT_PITCH, h, v);
+    double2 w[R1];
+    if (h < TPC) ct::dft2_back2<R1, R2, 1>(col, ZT_PITCH, h, w);
     const int l = m + ZT_COLS * c + j;
-    if (h < R1 && l <= a.lmax) {
+    if (h < R2 && l <= a.lmax) {
 #pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2)
-        a.dout[(size_t)(a.mbase[m] - m) + (size_t)(h + R1 * k2) * a.nlm + l] = v[k2];
+      for (int b = 0; b < R1; ++b)
+        a.dout[(size_t)(a.mbase[m] - m) + (size_t)(h + R2 * b) * a.nlm + l] = w[b];
     }
   }
 }

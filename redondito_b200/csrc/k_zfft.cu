@@ -184,23 +184,23 @@ __global__ void __launch_bounds__(ZTHREADS) zfft_kernel(ZArgs a) {
 // in zfft_kernel (same loads and continuation, the inverse's input in
 // natural order).  A plain transform is the two register steps, its results
 // stored from registers; the spectral modes run the forward steps, multiply
-// in registers, put the spectrum back in natural order and run the inverse
-// steps.
-// The columns per CTA are those launch_zfft_io picks by default for the
-// length (32 KB slabs), fixed at compile time; other choices take the radix
-// kernel.  Registers are held to 80 per thread for the plain transforms
-// (six CTAs of 128 threads per SM at nz 256; 1.66 against 1.68 ms for eight
-// transforms with five) and 128 for the spectral modes (four).
+// in registers and go back from there (dft2_back1/2: one more exchange).
+// About 128 threads per CTA (8 columns at nz 96 and above), 80 registers: the
+// kernels wait on loads and barriers, not on HBM or the FP64 pipe (29% busy
+// in the derivative), so many small CTAs overlap best.  Derivative and D_l of
+// 32896 columns: nz 96 55 and 64 -> 36 and 48 us, nz 128 53 and 66 -> 43 and
+// 64 us, against the spectrum put back in natural order between two full
+// splits, 128-148 registers and 16 columns.
 __host__ __device__ constexpr int z2_lb(int nz) {
-  int lb = 64;
-  while (lb > 1 && lb * nz > ZMAXCOL / 2) lb >>= 1;
+  int lb = 32;
+  while (lb > 8 && lb * ct::split2_tpc(nz) > 128) lb >>= 1;
   return lb;
 }
 template <int MODE, int NZ, int TPC>
 struct Z2Geo {
   static constexpr int LB = z2_lb(NZ), THREADS = LB * TPC;
   static constexpr bool PLAIN = MODE == Z_FWD || MODE == Z_INV;
-  static constexpr int RPT = PLAIN ? 84 : 128;
+  static constexpr int RPT = 84;
   static constexpr int MINB = 65536 / (THREADS * RPT) > 1 ? 65536 / (THREADS * RPT) : 1;
 };
 
@@ -216,16 +216,11 @@ __device__ __forceinline__ void zfft2_body(const ZArgs& a, int blk) {
   const int nlm = a.nlm, tid = threadIdx.x, lm0 = blk * LB;
   const bool cont = MODE != Z_INV && a.C > 0;
   const int nload = cont ? a.N : NZ;
-  double2* orig = sm + (size_t)LB * NZ;  // D_l keeps the input column for the l(l+1)/r^2 term
-  for (int idx = tid; idx < nload * LB; idx += nthreads) {
+  // D_l keeps the whole input column (in, every row) for its l(l+1)/r^2 term
+  double2* in = MODE == Z_DLR ? sm + (size_t)LB * NZ : sm;
+  for (int idx = tid; idx < (MODE == Z_DLR ? NZ : nload) * LB; idx += nthreads) {
     const int r = idx / LB, c = idx - r * LB, lm = lm0 + c;
-    zload<IO>(a, sm + idx, (size_t)r * nlm + lm, lm < nlm);
-  }
-  if (MODE == Z_DLR) {
-    for (int idx = tid; idx < NZ * LB; idx += nthreads) {
-      const int r = idx / LB, c = idx - r * LB, lm = lm0 + c;
-      zload<IO>(a, orig + idx, (size_t)r * nlm + lm, lm < nlm);
-    }
+    zload<IO>(a, in + idx, (size_t)r * nlm + lm, lm < nlm);
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -234,49 +229,64 @@ __device__ __forceinline__ void zfft2_body(const ZArgs& a, int blk) {
     const int C = a.C, d = a.d, N = a.N;
     for (int idx = tid; idx < C * LB; idx += nthreads) {
       const int ii = idx / LB, c = idx - ii * LB;
-      sm[(N + ii) * LB + c] = fc_cont_elem(a.dir, C, d, N, ii, sm + c, LB);
+      sm[(N + ii) * LB + c] = fc_cont_elem(a.dir, C, d, N, ii, in + c, LB);
     }
     __syncthreads();
   }
   const int c = tid % LB, h = tid / LB, lm = lm0 + c;
   double2* col = sm + c;
-  ct::dft2_step1<R1, R2, SG>(col, LB, h, a.fd.tw);
+  if constexpr (MODE == Z_DLR) {
+    // step 1 with the physical rows from the kept column
+    if (h < R2) {
+      double2 w[R1];
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) {
+        const int r = h + R2 * n1;
+        w[n1] = r < nload ? in[r * LB + c] : col[r * LB];
+      }
+      ct::dft2_put1<R1, R2, SG>(w, col, LB, h, a.fd.tw);
+    }
+  } else {
+    ct::dft2_step1<R1, R2, SG>(col, LB, h, a.fd.tw);
+  }
   __syncthreads();
   double2 v[R2];
   ct::dft2_step2<R1, R2, SG>(col, LB, h, v);
-  if constexpr (!PLAIN) {
-    // X[k] / nz times (i kz)^p or the filter, k = h + R1 k2; back in natural
-    // order once every thread has read its step-2 slots; then the inverse
-    __syncthreads();
+  if constexpr (PLAIN) {
+    if (h < R1 && lm < nlm) {
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2)
+        zstore<IO>(a, (size_t)(h + R1 * k2) * nlm + lm, MODE == Z_FWD ? div_nz(v[k2], NZ) : v[k2]);
+    }
+  } else {
+    // X[k] / nz times (i kz)^p or the filter, k = h + R1 k2, in registers, and back
     if (h < R1) {
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2) {
         const int k = h + R1 * k2;
-        double2 x = div_nz(v[k2], NZ);
-        if (MODE == Z_FILTER) x = cscale(x, a.filt[k]);
-        else x = cmul(a.kfac[k], x);
-        col[k * LB] = x;
+        const double2 x = div_nz(v[k2], NZ);
+        v[k2] = MODE == Z_FILTER ? cscale(x, a.filt[k]) : cmul(a.kfac[k], x);
       }
     }
+    ct::dft2_back1<R1, R2, 1>(v, col, LB, h, a.fd.tw);
     __syncthreads();
-    ct::dft2_step1<R1, R2, 1>(col, LB, h, a.fd.tw);
-    __syncthreads();
-    ct::dft2_step2<R1, R2, 1>(col, LB, h, v);
-  }
-  if (h < R1 && lm < nlm) {
+    double2 w[R1];
+    ct::dft2_back2<R1, R2, 1>(col, LB, h, w);
+    if (h < R2 && lm < nlm) {
 #pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) {
-      const int r = h + R1 * k2;
-      double2 x = MODE == Z_FWD ? div_nz(v[k2], NZ) : v[k2];
-      if (MODE == Z_DLR) {
-        // b = b + z^-2 * (-l(l+1) a)   (laplang, multr(-2), saxpby_c)
-        const double lf = -(double)(a.ell[lm] * (a.ell[lm] + 1));
-        const double2 o = orig[r * LB + c];
-        const double zi = a.zinv2[r];
-        x.x = x.x + zi * (lf * o.x);
-        x.y = x.y + zi * (lf * o.y);
+      for (int b = 0; b < R1; ++b) {
+        const int r = h + R2 * b;
+        double2 x = w[b];
+        if (MODE == Z_DLR) {
+          // b = b + z^-2 * (-l(l+1) a)   (laplang, multr(-2), saxpby_c)
+          const double lf = -(double)(a.ell[lm] * (a.ell[lm] + 1));
+          const double2 o = in[r * LB + c];
+          const double zi = a.zinv2[r];
+          x.x = x.x + zi * (lf * o.x);
+          x.y = x.y + zi * (lf * o.y);
+        }
+        zstore<IO>(a, (size_t)r * nlm + lm, x);
       }
-      zstore<IO>(a, (size_t)r * nlm + lm, x);
     }
   }
 }
@@ -424,16 +434,17 @@ int launch_ct(const ZArgs& a, int nblocks, size_t smem, cudaStream_t st) {
 
 #define Z_SIZES(X) X(16) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(512)
 
-// the lengths that take the two-step split
-bool zsplit_length(int nz) {
+// the two-step kernel's columns per CTA for the lengths that take it, else 0
+int zsplit_lb(int nz) {
   switch (nz) {
 #define CASE(n) \
-  case n: return ct::split2_r1(n) > 0;
+  case n: return std::integral_constant<int, (ct::split2_r1(n) > 0 ? z2_lb(n) : 0)>::value;
     Z_SIZES(CASE)
 #undef CASE
   }
-  return false;
+  return 0;
 }
+bool zsplit_length(int nz) { return zsplit_lb(nz) > 0; }
 
 bool ct_length(int nz) {
   switch (nz) {
@@ -508,6 +519,7 @@ int make_zargs(const sph_plan* p, int mode, const void* in, void* out, int order
   while (LB > 1 && LB * p->nz > ZMAXCOL / 2) LB >>= 1;
   // a tuned width, except for the lengths with the two-step split, whose
   // kernel is compiled for the default width
+  if (zsplit_length(p->nz)) LB = zsplit_lb(p->nz);
   if (!ct_length(p->nz)) LB = zgen_lb(p->nz, p->nlmv);
   if (p->tile_lb && !zsplit_length(p->nz)) LB = p->tile_lb;
   if (LB * p->nz > ZMAXCOL) return SPH_EINVAL;
@@ -585,7 +597,7 @@ int zfwd_group_prepare(const std::vector<ZJob>& jobs, ZGroupLaunch* g, std::vect
     int nb = 0;
     if (!p || !jobs[k].spec || !zsplit_length(p->nz) ||
         make_zargs(p, Z_FWD, jobs[k].spec, jobs[k].spec, 0, jobs[k].cont, &a, &nb) != SPH_OK || nb < 1 ||
-        a.LB != z2_lb(p->nz)) {
+        a.LB != zsplit_lb(p->nz)) {
       rest->push_back(k);
       continue;
     }
@@ -707,6 +719,7 @@ extern "C" int sph_derivr_noalloc(const double* a, double* b, int nlm, int nz, i
   // the column blocks of the plan path (so that both run the same kernel)
   while (LB > 1 && LB * nz > ZMAXCOL / 2) LB >>= 1;
   if (LB * nz > ZMAXCOL) return SPH_EINVAL;
+  if (zsplit_length(nz)) LB = zsplit_lb(nz);
   if (!ct_length(nz)) LB = zgen_lb(nz, nlm);
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return SPH_ECUDA;
