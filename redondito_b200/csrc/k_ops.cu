@@ -256,34 +256,39 @@ __global__ void bc_fast_kernel(double2* phi, const double2* __restrict__ w, cons
   }
 }
 
-// QST potentials of u and curl u: out = sc * z^rpow * (l(l+1) if lfac) * in
-__global__ void qst_scale_kernel(const double2* __restrict__ a, double2* __restrict__ b,
-                                 const double* __restrict__ z, const int* __restrict__ ell, int rpow,
-                                 int lfac, double sc, int nlm, size_t n) {
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    int l = ell[q % nlm];
-    double f = sc * pow(z[q / nlm], (double)rpow) * (lfac ? (double)(l * (l + 1)) : 1.0);
-    b[q] = cscale(a[q], f);
-  }
+// the toroidal potential of curl u: b = -a / r
+__global__ void neg_over_r_kernel(const double2* __restrict__ a, double2* __restrict__ b,
+                                  const double* __restrict__ zinv, int nlm) {
+  const double f = -zinv[blockIdx.y];
+  const size_t row = (size_t)blockIdx.y * nlm;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nlm; q += gridDim.x * blockDim.x)
+    b[row + q] = cscale(a[row + q], f);
 }
 
-// 0.5 * sum_k c_k r_k^2 dz sum_{j,i} w_i (2 pi/nphi) |u|^2 over k < N (FP64)
-__global__ void energy_kernel(const double* __restrict__ ur, const double* __restrict__ ut,
-                              const double* __restrict__ up, const double* __restrict__ w,
-                              const double* __restrict__ z, int nlat, int nphi, int N, double scale,
-                              double* acc) {
+// prodvec on the physical planes and, from the same reads, the energy
+// 0.5 * sum_k c_k r_k^2 dz sum_{j,i} w_i (2 pi/nphi) |A|^2 (FP64): one pass of
+// 9 arrays over N planes (the two kernels read and wrote 12 over nz)
+__global__ void __launch_bounds__(EW_THREADS)
+    prodvec_energy_kernel(const double* __restrict__ ar, const double* __restrict__ at, const double* __restrict__ ap,
+                          const double* __restrict__ br, const double* __restrict__ bt, const double* __restrict__ bp,
+                          double* cr, double* ct, double* cp, const double* __restrict__ w,
+                          const double* __restrict__ z, int nlat, int nphi, int N, double scale, double* acc) {
   __shared__ double red[EW_THREADS / 32];
-  const size_t plane = (size_t)nlat * nphi;
-  const size_t n = plane * N;
+  const int half = nlat / 2, n = half * nphi;  // pairs of nodes of one plane
+  const size_t plane = (size_t)n * blockIdx.y;
+  auto ld = [&](const double* x, int q) { return __ldg(reinterpret_cast<const double2*>(x) + plane + q); };
+  auto st = [&](double* x, int q, double2 v) { reinterpret_cast<double2*>(x)[plane + q] = v; };
   double s = 0.0;
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
-    int k = (int)(q / plane);
-    int i = (int)(q % nlat);
-    double ck = (k == 0 || k == N - 1) ? 0.5 : 1.0;
-    double rk = z[k];
-    double v = ur[q] * ur[q] + ut[q] * ut[q] + up[q] * up[q];
-    s += ck * rk * rk * w[i] * v;
+  for (int q = blockIdx.x * EW_THREADS + threadIdx.x; q < n; q += gridDim.x * EW_THREADS) {
+    const double2 xr = ld(ar, q), xt = ld(at, q), xp = ld(ap, q), yr = ld(br, q), yt = ld(bt, q), yp = ld(bp, q);
+    st(cr, q, make_double2(xt.x * yp.x - xp.x * yt.x, xt.y * yp.y - xp.y * yt.y));
+    st(ct, q, make_double2(xp.x * yr.x - xr.x * yp.x, xp.y * yr.y - xr.y * yp.y));
+    st(cp, q, make_double2(xr.x * yt.x - xt.x * yr.x, xr.y * yt.y - xt.y * yr.y));
+    const double2 wi = __ldg(reinterpret_cast<const double2*>(w) + q % half);
+    s += wi.x * (xr.x * xr.x + xt.x * xt.x + xp.x * xp.x) + wi.y * (xr.y * xr.y + xt.y * xt.y + xp.y * xp.y);
   }
+  const int k = blockIdx.y;
+  s *= ((k == 0 || k == N - 1) ? 0.5 : 1.0) * z[k] * z[k];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -408,22 +413,22 @@ int launch_bc_fast_rows(const sph_plan* p, double2* phi, const double2* w, cudaS
   return SPH_OK;
 }
 
-int launch_qst_scale(const sph_plan* p, const double2* in, double2* out, int rpow, int lfac, double sc,
-                     cudaStream_t st) {
-  size_t n = spec_elems(p);
+int launch_neg_over_r(const sph_plan* p, const double2* in, double2* out, cudaStream_t st) {
   TimedLaunch tl(p, T_OPS, st);
-  qst_scale_kernel<<<ew_blocks(n), EW_THREADS, 0, st>>>(in, out, p->d_z, p->d_ell, rpow, lfac, sc, p->nlm, n);
+  const dim3 grid(std::min((p->nlm + EW_THREADS - 1) / EW_THREADS, 64), p->nz);
+  neg_over_r_kernel<<<grid, EW_THREADS, 0, st>>>(in, out, p->zinv, p->nlm);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
 
-int launch_energy(const sph_plan* p, const double* ur, const double* ut, const double* up, double* acc,
-                  cudaStream_t st) {
-  size_t n = (size_t)p->nlat * p->nphi * p->N;
-  double scale = 0.5 * p->dz * 2.0 * 3.14159265358979323846 / p->nphi;
+int launch_prodvec_energy(const sph_plan* p, double* const* A, double* const* B, double* const* C, double* acc,
+                          cudaStream_t st) {
+  const double scale = 0.5 * p->dz * 2.0 * 3.14159265358979323846 / p->nphi;
+  const int n = p->nlat / 2 * p->nphi;
   TimedLaunch tl(p, T_OPS, st);
-  energy_kernel<<<ew_blocks(n), EW_THREADS, 0, st>>>(ur, ut, up, p->wfull, p->d_z, p->nlat, p->nphi, p->N,
-                                                     scale, acc);
+  const dim3 grid(std::max(1, std::min((n + EW_THREADS - 1) / EW_THREADS, 32)), p->N);
+  prodvec_energy_kernel<<<grid, EW_THREADS, 0, st>>>(A[0], A[1], A[2], B[0], B[1], B[2], C[0], C[1], C[2], p->wfull,
+                                                     p->d_z, p->nlat, p->nphi, p->N, scale, acc);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }

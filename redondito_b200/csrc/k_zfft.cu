@@ -47,7 +47,18 @@ struct ZArgs {
   const double* zinv2;    // nz
   const int* ell;         // nlm
   FftDesc fd;
+  // the passes of the nonlinear step (Z_POT, Z_RHS, Z_DLADD)
+  ZNlArgs nl;
+  const double *z, *zinv;  // r, 1/r
 };
+
+// modes that keep the whole input column (every row) beside the transform's
+constexpr bool zkeep(int mode) { return mode == Z_DLR || mode == Z_POT || mode == Z_DLADD; }
+
+// The output of row r, column lm (at idx) of a spectral mode from the
+// transformed value x and the kept input o.
+template <int MODE, int IO>
+__device__ __forceinline__ void zspectral_store(const ZArgs& a, int r, int lm, size_t idx, double2 x, double2 o);
 
 // 16-byte global -> shared copy that lands asynchronously; src_bytes 0
 // writes zeros (src is then not read but must be a valid address)
@@ -85,6 +96,39 @@ __device__ __forceinline__ void zstore(const ZArgs& a, size_t idx, double2 v) {
     static_cast<float2*>(a.out)[idx] = make_float2((float)v.x, (float)v.y);
   else
     static_cast<double2*>(a.out)[idx] = v;
+}
+
+template <int MODE, int IO>
+__device__ __forceinline__ void zspectral_store(const ZArgs& a, int r, int lm, size_t idx, double2 x, double2 o) {
+  if constexpr (MODE == Z_DLR || MODE == Z_DLADD) {
+    // b = b + z^-2 * (-l(l+1) a)   (laplang, multr(-2), saxpby_c)
+    const double lf = -(double)(a.ell[lm] * (a.ell[lm] + 1));
+    const double zi = a.zinv2[r];
+    x.x = x.x + zi * (lf * o.x);
+    x.y = x.y + zi * (lf * o.y);
+  }
+  if constexpr (MODE == Z_DLADD) {
+    x = cscale(x, a.nl.nu);
+    if (!a.nl.by_r || r < a.N) {
+      const double f = a.nl.by_r ? a.z[r] : 1.0;
+      const double2 v = __ldg(a.nl.add + idx);
+      x = make_double2(f * v.x + x.x, f * v.y + x.y);
+    }
+    if (a.nl.base) {
+      const double2 v = __ldg(a.nl.base + idx);
+      x = make_double2(v.x + a.nl.c * x.x, v.y + a.nl.c * x.y);
+    }
+  }
+  if constexpr (MODE == Z_RHS) {
+    if (r < a.N) x = csub(x, __ldg(a.nl.q + idx));
+  }
+  if constexpr (MODE == Z_POT) {
+    const double zi = a.zinv[r];
+    a.nl.q[idx] = cscale(o, a.zinv2[r] * (double)(a.ell[lm] * (a.ell[lm] + 1)));
+    if (a.nl.t) a.nl.t[idx] = cscale(o, zi);
+    x = cscale(x, zi);
+  }
+  zstore<IO>(a, idx, x);
 }
 
 template <int MODE, int CTN, int IO>
@@ -216,14 +260,16 @@ __device__ __forceinline__ void zfft2_body(const ZArgs& a, int blk) {
   const int nlm = a.nlm, tid = threadIdx.x, lm0 = blk * LB;
   const bool cont = MODE != Z_INV && a.C > 0;
   const int nload = cont ? a.N : NZ;
-  // D_l keeps the whole input column (in, every row) for its l(l+1)/r^2 term
-  double2* in = MODE == Z_DLR ? sm + (size_t)LB * NZ : sm;
-  for (int idx = tid; idx < (MODE == Z_DLR ? NZ : nload) * LB; idx += nthreads) {
+  constexpr bool KEEP = zkeep(MODE);
+  double2* in = KEEP ? sm + (size_t)LB * NZ : sm;
+  for (int idx = tid; idx < (KEEP ? NZ : nload) * LB; idx += nthreads) {
     const int r = idx / LB, c = idx - r * LB, lm = lm0 + c;
     zload<IO>(a, in + idx, (size_t)r * nlm + lm, lm < nlm);
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if constexpr (MODE == Z_RHS)  // r x, each thread the elements it copied
+    for (int idx = tid; idx < nload * LB; idx += nthreads) sm[idx] = cscale(sm[idx], a.z[idx / LB]);
   __syncthreads();
   if (cont) {  // as in zfft_kernel
     const int C = a.C, d = a.d, N = a.N;
@@ -235,7 +281,7 @@ __device__ __forceinline__ void zfft2_body(const ZArgs& a, int blk) {
   }
   const int c = tid % LB, h = tid / LB, lm = lm0 + c;
   double2* col = sm + c;
-  if constexpr (MODE == Z_DLR) {
+  if constexpr (KEEP) {
     // step 1 with the physical rows from the kept column
     if (h < R2) {
       double2 w[R1];
@@ -276,16 +322,7 @@ __device__ __forceinline__ void zfft2_body(const ZArgs& a, int blk) {
 #pragma unroll
       for (int b = 0; b < R1; ++b) {
         const int r = h + R2 * b;
-        double2 x = w[b];
-        if (MODE == Z_DLR) {
-          // b = b + z^-2 * (-l(l+1) a)   (laplang, multr(-2), saxpby_c)
-          const double lf = -(double)(a.ell[lm] * (a.ell[lm] + 1));
-          const double2 o = in[r * LB + c];
-          const double zi = a.zinv2[r];
-          x.x = x.x + zi * (lf * o.x);
-          x.y = x.y + zi * (lf * o.y);
-        }
-        zstore<IO>(a, (size_t)r * nlm + lm, x);
+        zspectral_store<MODE, IO>(a, r, lm, (size_t)r * nlm + lm, w[b], KEEP ? in[r * LB + c] : w[b]);
       }
     }
   }
@@ -325,18 +362,19 @@ __global__ void __launch_bounds__(ZTHREADS, 2) zfft_gen_kernel(ZArgs a, int lg) 
   const int LB = 1 << lg, nz = a.nz, nlm = a.nlm, lm0 = blockIdx.x << lg, tid = threadIdx.x;
   const bool cont = MODE != Z_INV && a.C > 0;
   const int nload = cont ? a.N : nz, total = nz << lg;
-  double2* orig = sm + 2 * total;  // D_l keeps the input column for the l(l+1)/r^2 term
-  for (int idx = tid; idx < nload << lg; idx += ZTHREADS) {
+  constexpr bool KEEP = zkeep(MODE);
+  double2* orig = sm + 2 * total;
+  for (int idx = tid; idx < (KEEP ? total : nload << lg); idx += ZTHREADS) {
     const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
-    zload<IO>(a, sm + idx, (size_t)r * nlm + lm, lm < nlm);
+    zload<IO>(a, (KEEP ? orig : sm) + idx, (size_t)r * nlm + lm, lm < nlm);
   }
-  if (MODE == Z_DLR)
-    for (int idx = tid; idx < total; idx += ZTHREADS) {
-      const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
-      zload<IO>(a, orig + idx, (size_t)r * nlm + lm, lm < nlm);
-    }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  // each thread the elements it copied: the transform's copy of a kept
+  // column, or r x
+  if constexpr (KEEP || MODE == Z_RHS)
+    for (int idx = tid; idx < nload << lg; idx += ZTHREADS)
+      sm[idx] = KEEP ? orig[idx] : cscale(sm[idx], a.z[idx >> lg]);
   __syncthreads();
   if (cont) {  // as in zfft_kernel
     for (int idx = tid; idx < a.C << lg; idx += ZTHREADS) {
@@ -347,7 +385,7 @@ __global__ void __launch_bounds__(ZTHREADS, 2) zfft_gen_kernel(ZArgs a, int lg) 
   }
   constexpr int SG = MODE == Z_INV ? 1 : -1;  // first transform's sign
   double2* x = fg::run<SG>(sm, sm + total, nz, a.fd.gf, 0, a.fd.ng, lg, a.fd.tw);
-  if constexpr (MODE == Z_DERIV || MODE == Z_FILTER || MODE == Z_DLR) {
+  if constexpr (MODE != Z_FWD && MODE != Z_INV) {
     for (int idx = tid; idx < total; idx += ZTHREADS) {
       const int k = idx >> lg;
       const double2 v = div_nz(x[idx], nz);
@@ -359,16 +397,9 @@ __global__ void __launch_bounds__(ZTHREADS, 2) zfft_gen_kernel(ZArgs a, int lg) 
   for (int idx = tid; idx < total; idx += ZTHREADS) {
     const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
     if (lm >= nlm) continue;
-    double2 v = MODE == Z_FWD ? div_nz(x[idx], nz) : x[idx];
-    if (MODE == Z_DLR) {
-      // b = b + z^-2 * (-l(l+1) a)   (laplang, multr(-2), saxpby_c)
-      const double lf = -(double)(a.ell[lm] * (a.ell[lm] + 1));
-      const double2 o = orig[idx];
-      const double zi = a.zinv2[r];
-      v.x = v.x + zi * (lf * o.x);
-      v.y = v.y + zi * (lf * o.y);
-    }
-    zstore<IO>(a, (size_t)r * nlm + lm, v);
+    const size_t o = (size_t)r * nlm + lm;
+    if constexpr (MODE == Z_FWD || MODE == Z_INV) zstore<IO>(a, o, MODE == Z_FWD ? div_nz(x[idx], nz) : x[idx]);
+    else zspectral_store<MODE, IO>(a, r, lm, o, x[idx], KEEP ? orig[idx] : x[idx]);
   }
 }
 
@@ -394,8 +425,25 @@ int launch_gen(const ZArgs& a, cudaStream_t st) {
     return SPH_ECUDA;
   int lg = 0;
   while ((1 << lg) < a.LB) ++lg;
-  const size_t smem = ((size_t)a.nz << lg) * sizeof(double2) * (MODE == Z_DLR ? 3 : 2);
+  const size_t smem = ((size_t)a.nz << lg) * sizeof(double2) * (zkeep(MODE) ? 3 : 2);
   zfft_gen_kernel<MODE, IO><<<(a.nlm + a.LB - 1) / a.LB, ZTHREADS, smem, st>>>(a, lg);
+  SPH_LAUNCH_OK();
+  return SPH_OK;
+}
+
+template <int MODE, int R1, int R2, int IO>
+int launch_split(const ZArgs& a, int nblocks, cudaStream_t st) {
+  using GZ = Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>;
+  static DeviceOnce once;
+  if (!once.run([] {
+        return cudaFuncSetAttribute(zfft2_kernel<MODE, R1, R2, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    200 * 1024) == cudaSuccess &&
+               cudaFuncSetAttribute(zfft2_kernel<MODE, R1, R2, IO>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    100) == cudaSuccess;
+      }))
+    return SPH_ECUDA;
+  const size_t smem = (size_t)GZ::LB * R1 * R2 * sizeof(double2) * (zkeep(MODE) ? 2 : 1);
+  zfft2_kernel<MODE, R1, R2, IO><<<nblocks, GZ::THREADS, smem, st>>>(a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -413,19 +461,7 @@ int launch_ct(const ZArgs& a, int nblocks, size_t smem, cudaStream_t st) {
   if constexpr (CTN > 0 && ct::split2_r1(CTN) > 0) {
     constexpr int R1 = ct::split2_r1(CTN), R2 = CTN / R1;
     using GZ = Z2Geo<MODE, CTN, ct::split2_tpc(CTN)>;
-    if (a.LB == GZ::LB) {
-      static DeviceOnce once2;
-      if (!once2.run([] {
-            return cudaFuncSetAttribute(zfft2_kernel<MODE, R1, R2, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        200 * 1024) == cudaSuccess &&
-                   cudaFuncSetAttribute(zfft2_kernel<MODE, R1, R2, IO>,
-                                        cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
-          }))
-        return SPH_ECUDA;
-      zfft2_kernel<MODE, R1, R2, IO><<<nblocks, GZ::THREADS, smem, st>>>(a);
-      SPH_LAUNCH_OK();
-      return SPH_OK;
-    }
+    if (a.LB == GZ::LB) return launch_split<MODE, R1, R2, IO>(a, nblocks, st);
   }
   zfft_kernel<MODE, CTN, IO><<<nblocks, ZTHREADS, smem, st>>>(a);
   SPH_LAUNCH_OK();
@@ -525,7 +561,10 @@ int make_zargs(const sph_plan* p, int mode, const void* in, void* out, int order
   if (LB * p->nz > ZMAXCOL) return SPH_EINVAL;
   a.LB = LB;
   *nblocks = (p->nlmv + LB - 1) / LB;
-  if (mode == Z_DLR) a.kfac = p->kfac + (size_t)1 * p->nz;  // (i kz)^2
+  if (mode == Z_DLR || mode == Z_DLADD) a.kfac = p->kfac + (size_t)1 * p->nz;  // (i kz)^2
+  a.nl = {};
+  a.z = p->d_z;
+  a.zinv = p->zinv;
   return SPH_OK;
 }
 
@@ -547,6 +586,41 @@ int launch_zfft_io(const sph_plan* p, int mode, const void* in, void* out, int i
       return launch_mode_io<Z_DERIV>(a, io, nblocks, smem, st);
     case Z_FILTER: return launch_mode_io<Z_FILTER>(a, io, nblocks, smem, st);
     case Z_DLR: return launch_mode_io<Z_DLR>(a, io, nblocks, smem, st);
+  }
+  return SPH_EINVAL;
+}
+
+namespace {
+
+// the nonlinear step's passes: the two-step kernel for its lengths, the
+// general one for the others
+template <int MODE>
+int launch_nl(const ZArgs& a, int nblocks, cudaStream_t st) {
+  switch (a.nz) {
+#define CASE(n)                                                                                             \
+  case n:                                                                                                   \
+    if constexpr (ct::split2_r1(n) > 0)                                                                     \
+      return launch_split<MODE, std::max(1, ct::split2_r1(n)), n / std::max(1, ct::split2_r1(n)), ZIO_DD>(a, nblocks, st); \
+    break;
+    Z_SIZES(CASE)
+#undef CASE
+  }
+  return launch_gen<MODE, ZIO_DD>(a, st);
+}
+
+}  // namespace
+
+int launch_znl(const sph_plan* p, int mode, const double2* x, double2* out, const ZNlArgs& nl, cudaStream_t st) {
+  ZArgs a;
+  int nblocks = 0;
+  const int rc = make_zargs(p, mode, x, out, 1, true, &a, &nblocks);
+  if (rc != SPH_OK) return rc;
+  a.nl = nl;
+  TimedLaunch tl(p, T_ZFFT, st);
+  switch (mode) {
+    case Z_POT: return launch_nl<Z_POT>(a, nblocks, st);
+    case Z_RHS: return launch_nl<Z_RHS>(a, nblocks, st);
+    case Z_DLADD: return launch_nl<Z_DLADD>(a, nblocks, st);
   }
   return SPH_EINVAL;
 }

@@ -165,7 +165,7 @@ static int upload(T** dst, const T* src, size_t n) {
 
 // the read-only device tables of a plan (shared with its clones)
 static std::vector<void*> table_ptrs(const sph_plan* p) {
-  return {p->P, p->dP, p->mPs, p->wfold, p->wfull, p->d_dir, p->d_z, p->kfac, p->filt, p->zinv2, p->d_ell,
+  return {p->P, p->dP, p->mPs, p->wfold, p->wfull, p->d_dir, p->d_z, p->kfac, p->filt, p->zinv, p->zinv2, p->d_ell,
           p->d_mbase, p->twz, p->twphi, p->twzf, p->twphif, p->revz, p->revphi, p->twpz, p->twpphi, p->twpzf,
           p->twpphif, p->tw4f, p->tw4d, p->tilesA, p->tilesA32, p->tilesS, p->tilesS32, p->d_bplanes, p->d_toff};
 }
@@ -328,10 +328,11 @@ extern "C" int sph_plan_create(sph_plan** out, int lmax, int nlat, int nphi, int
       double im = (o % 4 == 1) ? 1 : (o % 4 == 3) ? -1 : 0;
       kf[(size_t)(o - 1) * nz + k] = make_double2(re * kp, im * kp);
     }
-  std::vector<double> filt(nz), zinv2(nz);
+  std::vector<double> filt(nz), zinv(nz), zinv2(nz);
   const double alpha = 16.0 * log(10.0);
   for (int k = 0; k < nz; ++k) {
     filt[k] = exp(-alpha * pow(2.0 * p->kz[k] / nz / p->Dkz, 100.0));
+    zinv[k] = 1.0 / p->z[k];
     zinv2[k] = 1.0 / (p->z[k] * p->z[k]);
   }
   std::vector<double2> twz, twp;
@@ -372,6 +373,7 @@ extern "C" int sph_plan_create(sph_plan** out, int lmax, int nlat, int nphi, int
   UP(p->d_z, p->z);
   UP(p->kfac, kf);
   UP(p->filt, filt);
+  UP(p->zinv, zinv);
   UP(p->zinv2, zinv2);
   UP(p->d_ell, p->ell);
   UP(p->d_mbase, p->mbase);
@@ -1218,50 +1220,64 @@ struct BoundaryPass {
   ~BoundaryPass() { p->bpass = 0; }
 };
 
+// Inside the NL step the angular transforms run on the physical planes
+// k < N only: u and curl u are used nowhere else, and N = u x curl u is zero
+// on the continuation planes, so its spectra are zero there (the radial
+// passes take those rows as zero instead of reading them).  At nz 128 with
+// C = 25 that is a fifth of the angular work.
+struct PhysicalPlanes {
+  sph_plan* p;
+  explicit PhysicalPlanes(sph_plan* p_) : p(p_) { p->nzv = p->N; }
+  ~PhysicalPlanes() { p->nzv = p->nz; }
+};
+
+// The right-hand sides into rz and rf, or, with Z0 and F0, the update
+// rz = Z0 + c rhs_z, rf = F0 + c rhs_phi.  rz may be Z, rf may be F.
 static int nl_rhs_impl(sph_plan* p, const double2* Z, const double2* W, const double2* F, double nu,
-                       double2* rz, double2* rf, cudaStream_t st) {
+                       double2* rz, double2* rf, const double2* Z0, const double2* F0, double c, cudaStream_t st) {
   BoundaryPass bp(p);
   double2 *s0 = p->sp[0], *s1 = p->sp[1], *s2 = p->sp[2], *s3 = p->sp[3], *s4 = p->sp[4];
   double* g[9];
   for (int i = 0; i < 9; ++i) g[i] = p->gr[i];
-  // u: Q = l(l+1) W/r^2, S = W'/r, T = Z/r
-  RC(launch_qst_scale(p, W, s0, -2, 1, 1.0, st));
-  RC(launch_zfft(p, Z_DERIV, W, s3, 1, st));
-  RC(launch_qst_scale(p, s3, s1, -1, 0, 1.0, st));
-  RC(launch_qst_scale(p, Z, s2, -1, 0, 1.0, st));
-  RC(sph_fftp2d_qst_to_vec(p, (double*)s0, (double*)s1, (double*)s2, g[0], g[1], g[2], st));
-  // curl u: Q = l(l+1) Z/r^2, S = Z'/r, T = -phi/r
-  RC(launch_qst_scale(p, Z, s0, -2, 1, 1.0, st));
-  RC(launch_zfft(p, Z_DERIV, Z, s3, 1, st));
-  RC(launch_qst_scale(p, s3, s1, -1, 0, 1.0, st));
-  RC(launch_qst_scale(p, F, s2, -1, 0, -1.0, st));
-  RC(sph_fftp2d_qst_to_vec(p, (double*)s0, (double*)s1, (double*)s2, g[3], g[4], g[5], st));
-  SPH_CUDA_OK(cudaMemsetAsync(p->energy, 0, sizeof(double), st));
-  RC(launch_energy(p, g[0], g[1], g[2], p->energy, st));
-  // N = u x curl u, back to (Q, S, T)
-  const double* A[3] = {g[0], g[1], g[2]};
-  const double* B[3] = {g[3], g[4], g[5]};
-  double* Cc[3] = {g[6], g[7], g[8]};
-  RC(launch_prodvec(p, A, B, Cc, st));
-  RC(sph_fftp2d_vec_to_qst(p, g[6], g[7], g[8], (double*)s0, (double*)s1, (double*)s2, st));
+  // u: Q = l(l+1) W/r^2, S = W'/r, T = Z/r;  curl u: Q = l(l+1) Z/r^2, S = Z'/r, T = -phi/r
+  ZNlArgs a = {};
+  a.q = s0;
+  RC(launch_znl(p, Z_POT, W, s1, a, st));
+  a.q = s3;
+  a.t = s2;
+  RC(launch_znl(p, Z_POT, Z, s4, a, st));
+  {
+    PhysicalPlanes phys(p);
+    RC(sph_fftp2d_qst_to_vec(p, (double*)s0, (double*)s1, (double*)s2, g[0], g[1], g[2], st));
+    RC(launch_neg_over_r(p, F, s2, st));
+    RC(sph_fftp2d_qst_to_vec(p, (double*)s3, (double*)s4, (double*)s2, g[3], g[4], g[5], st));
+    SPH_CUDA_OK(cudaMemsetAsync(p->energy, 0, sizeof(double), st));
+    // N = u x curl u, back to (Q, S, T)
+    RC(launch_prodvec_energy(p, g, g + 3, g + 6, p->energy, st));
+    RC(sph_fftp2d_vec_to_qst(p, g[6], g[7], g[8], (double*)s0, (double*)s1, (double*)s2, st));
+  }
   // rhs_z = r T_N + nu D_l Z
-  RC(launch_multr(p, s2, s4, 1, st));
-  RC(launch_zfft(p, Z_DLR, Z, s3, 2, st));
-  RC(launch_saxpby(p, (double*)rz, (const double*)s4, 1.0, (const double*)s3, nu, 2 * spec_elems(p), st));
-  // rhs_phi = (r S_N)' - Q_N + nu D_l phi
-  RC(launch_multr(p, s1, s4, 1, st));
-  RC(launch_zfft(p, Z_DERIV, s4, s3, 1, st));
-  RC(launch_saxpby(p, (double*)rf, (const double*)s3, 1.0, (const double*)s0, -1.0, 2 * spec_elems(p), st));
-  RC(launch_zfft(p, Z_DLR, F, s4, 2, st));
-  RC(launch_saxpby(p, (double*)rf, (const double*)rf, 1.0, (const double*)s4, nu, 2 * spec_elems(p), st));
-  return SPH_OK;
+  a = {};
+  a.nu = nu;
+  a.c = c;
+  a.add = s2;
+  a.by_r = 1;
+  a.base = Z0;
+  RC(launch_znl(p, Z_DLADD, Z, rz, a, st));
+  // rhs_phi = (r S_N)' - Q_N + nu D_l phi, its first part in s3
+  a.q = s0;
+  RC(launch_znl(p, Z_RHS, s1, s3, a, st));
+  a.add = s3;
+  a.by_r = 0;
+  a.base = F0;
+  return launch_znl(p, Z_DLADD, F, rf, a, st);
 }
 
 extern "C" int sph_nl_rhs(sph_plan* p, const double* Z, const double* W, const double* phi, double nu,
                           double* rhs_z, double* rhs_phi, double* energy, void* s) {
   if (!p || !Z || !W || !phi || !rhs_z || !rhs_phi || !slab_whole(p)) return SPH_EINVAL;
   if (!p->bc_ready) return SPH_ENOTREADY;
-  RC(nl_rhs_impl(p, CD2(Z), CD2(W), CD2(phi), nu, D2(rhs_z), D2(rhs_phi), ST(s)));
+  RC(nl_rhs_impl(p, CD2(Z), CD2(W), CD2(phi), nu, D2(rhs_z), D2(rhs_phi), nullptr, nullptr, 1.0, ST(s)));
   if (energy) {
     SPH_CUDA_OK(cudaMemcpyAsync(energy, p->energy, sizeof(double), cudaMemcpyDeviceToHost, ST(s)));
     SPH_CUDA_OK(cudaStreamSynchronize(ST(s)));
@@ -1275,14 +1291,13 @@ extern "C" int sph_rk3_step(sph_plan* p, double* Z, double* W, double* phi, doub
   if (!p->bc_ready) return SPH_ENOTREADY;
   cudaStream_t st = ST(s);
   const size_t bytes = spec_elems(p) * sizeof(double2);
-  double2 *Z0 = p->sp[5], *F0 = p->sp[6], *rz = p->sp[7], *rf = p->sp[8], *e0 = p->sp[9];
+  double2 *Z0 = p->sp[5], *F0 = p->sp[6], *e0 = p->sp[9];
   SPH_CUDA_OK(cudaMemcpyAsync(Z0, Z, bytes, cudaMemcpyDeviceToDevice, st));
   SPH_CUDA_OK(cudaMemcpyAsync(F0, phi, bytes, cudaMemcpyDeviceToDevice, st));
   for (int o = 3; o >= 1; --o) {
-    RC(nl_rhs_impl(p, CD2(Z), CD2(W), CD2(phi), nu, rz, rf, st));
+    // Z = Z0 + dt/o rhs_z, phi = F0 + dt/o rhs_phi, written over Z and phi
+    RC(nl_rhs_impl(p, CD2(Z), CD2(W), CD2(phi), nu, D2(Z), D2(phi), Z0, F0, dt / o, st));
     if (o == 3) SPH_CUDA_OK(cudaMemcpyAsync(e0, p->energy, sizeof(double), cudaMemcpyDeviceToDevice, st));
-    RC(launch_saxpby(p, Z, (const double*)Z0, 1.0, (const double*)rz, dt / o, 2 * spec_elems(p), st));
-    RC(launch_saxpby(p, phi, (const double*)F0, 1.0, (const double*)rf, dt / o, 2 * spec_elems(p), st));
     RC(sph_v_imposebc(p, Z, phi, W, st));
   }
   if (energy) {

@@ -100,6 +100,7 @@ struct sph_plan {
   double* d_z = nullptr;    // [nz]
   double2* kfac = nullptr;  // [4][nz] (i kz)^p for p = 1..4
   double* filt = nullptr;   // [nz] exponential filter factors
+  double* zinv = nullptr;   // [nz] 1/z
   double* zinv2 = nullptr;  // [nz] 1/z^2
   int* d_ell = nullptr;     // [nlm]
   int* d_mbase = nullptr;   // [lmax+2]
@@ -265,7 +266,7 @@ __device__ __forceinline__ double2 cmul_si(double2 a, int sign) {
 
 // ---------------------------------------------------------------- launchers
 // z transforms (k_zfft.cu)
-enum ZMode { Z_FWD = 0, Z_INV = 1, Z_DERIV = 2, Z_FILTER = 3, Z_DLR = 4 };
+enum ZMode { Z_FWD = 0, Z_INV = 1, Z_DERIV = 2, Z_FILTER = 3, Z_DLR = 4, Z_POT = 5, Z_RHS = 6, Z_DLADD = 7 };
 // cont = false: the planes past N are taken as given (already continued)
 int launch_zfft(const sph_plan* p, int mode, const double2* in, double2* out, int order,
                 cudaStream_t st, bool cont = true);
@@ -275,6 +276,21 @@ int launch_zfft(const sph_plan* p, int mode, const double2* in, double2* out, in
 enum { ZIO_DD = 0, ZIO_FF = 1, ZIO_DF = 2, ZIO_FD = 3 };
 int launch_zfft_io(const sph_plan* p, int mode, const void* in, void* out, int io, int order, cudaStream_t st,
                    bool cont = true);
+
+// The radial passes of the nonlinear step on whole fields: a derivative with
+// the pointwise factors and sums around it, one read of each operand.
+//   Z_POT    s = x'/r, q = l(l+1) x/r^2, t = x/r (t may be null)
+//   Z_RHS    out = (r x)' - q                         (q zero for rows >= N)
+//   Z_DLADD  out = base + c (f add + nu D_l x)  with f = r for rows < N and 0
+//            past them (by_r) or f = 1; base null: out = f add + nu D_l x
+// out may be x or base.
+struct ZNlArgs {
+  double2 *q, *t;
+  const double2 *add, *base;
+  double c, nu;
+  int by_r;
+};
+int launch_znl(const sph_plan* p, int mode, const double2* x, double2* out, const ZNlArgs& nl, cudaStream_t st);
 
 // phi transforms (k_phifft.cu): grid fields -> folded coefficients and back
 int launch_phi_fwd(const sph_plan* p, const double* const* grids, int nfields, cudaStream_t st);
@@ -304,10 +320,11 @@ int launch_bc_walls(const sph_plan* p, double2* tor, cudaStream_t st);
 int launch_reconstruct(const sph_plan* p, double2* f, int boun, int ord, const double* a, cudaStream_t st);
 int launch_invDl(const sph_plan* p, const double2* phi, double2* w, cudaStream_t st);
 int launch_bc_fast_rows(const sph_plan* p, double2* phi, const double2* w, cudaStream_t st);
-int launch_qst_scale(const sph_plan* p, const double2* in, double2* out, int rpow, int lfac,
-                     double sc, cudaStream_t st);
-int launch_energy(const sph_plan* p, const double* ur, const double* ut, const double* up,
-                  double* acc, cudaStream_t st);
+// out = -in / r
+int launch_neg_over_r(const sph_plan* p, const double2* in, double2* out, cudaStream_t st);
+// C = A x B on the physical planes and the kinetic energy of A, in one pass
+int launch_prodvec_energy(const sph_plan* p, double* const* A, double* const* B, double* const* C, double* acc,
+                          cudaStream_t st);
 
 // mixed precision (k_mixed.cu)
 int mixed_setup(sph_plan* p, const std::vector<double>& hP, const std::vector<double>& hdP,
