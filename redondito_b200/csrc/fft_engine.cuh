@@ -186,3 +186,77 @@ __device__ __forceinline__ void fft_dit(double2* buf, const FftDesc& fd, const F
     s *= R;
   }
 }
+
+// The same transforms with the primes' passes out of place between two
+// buffers, one thread per output instead of per butterfly (its R inputs and
+// outputs need no local memory, and a few columns fill a CTA).  Every output
+// is the sum fft_pass_generic forms, term by term, so the results are its
+// bits.  Each returns the buffer that holds them; b is not used where every
+// radix is 2, 3, 4 or 8.
+template <bool DIT>
+__device__ __noinline__ void fft_pass_outputs(double2* src, double2* dst, const FftGeom& g, int R, int s,
+                                              const double2* __restrict__ tw, int sign) {
+  const int n = g.n, L = R * s, nq = n / R, nb = g.batch * nq, tstep = n / L, wR = n / R;
+  if (DIT && s > 1) {
+    for (int i = threadIdx.x; i < nb * (R - 1); i += blockDim.x) {
+      int b, q;
+      bfly_index(g, i % nb, nq, b, q);
+      const int blk = q / s, j = q - blk * s, r = 1 + i / nb, o = g.addr(b, blk * L + j + r * s);
+      if (j > 0) src[o] = cmul(src[o], tw_load(tw, j * r * tstep, sign));
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < nb * R; i += blockDim.x) {
+    int b, q;
+    bfly_index(g, i % nb, nq, b, q);
+    const int blk = q / s, j = q - blk * s, e0 = blk * L + j, qq = i / nb;
+    double2 acc = src[g.addr(b, e0)];
+    int e = 0;
+    for (int r = 1; r < R; ++r) {
+      const double2 x = src[g.addr(b, e0 + r * s)];
+      e += qq;
+      if (e >= R) e -= R;
+      acc = cadd(acc, e ? cmul(x, tw_load(tw, e * wR, sign)) : x);
+    }
+    if (!DIT && j > 0 && qq > 0) acc = cmul(acc, tw_load(tw, j * qq * tstep, sign));
+    dst[g.addr(b, e0 + qq * s)] = acc;
+  }
+  __syncthreads();
+}
+
+__host__ __device__ __forceinline__ bool fft_inplace_radix(int R) { return R <= 4 || R == 8; }
+
+template <bool DIT>
+__device__ __forceinline__ void run_pass2(double2*& a, double2*& b, const FftGeom& g, int R, int s,
+                                          const double2* __restrict__ tw, int sign) {
+  switch (R) {
+    case 2: fft_pass<2, DIT>(a, g, s, tw, sign); break;
+    case 3: fft_pass<3, DIT>(a, g, s, tw, sign); break;
+    case 4: fft_pass<4, DIT>(a, g, s, tw, sign); break;
+    case 8: fft_pass<8, DIT>(a, g, s, tw, sign); break;
+    default: {
+      fft_pass_outputs<DIT>(a, b, g, R, s, tw, sign);
+      double2* t = a;
+      a = b;
+      b = t;
+    }
+  }
+}
+
+__device__ __forceinline__ double2* fft_dif2(double2* a, double2* b, const FftDesc& fd, const FftGeom& g, int sign) {
+  int s = fd.n;
+  for (int ip = 0; ip < fd.npass; ++ip) {
+    s /= fd.pass[ip].R;
+    run_pass2<false>(a, b, g, fd.pass[ip].R, s, fd.tw, sign);
+  }
+  return a;
+}
+
+__device__ __forceinline__ double2* fft_dit2(double2* a, double2* b, const FftDesc& fd, const FftGeom& g, int sign) {
+  int s = 1;
+  for (int ip = fd.npass - 1; ip >= 0; --ip) {
+    run_pass2<true>(a, b, g, fd.pass[ip].R, s, fd.tw, sign);
+    s *= fd.pass[ip].R;
+  }
+  return a;
+}

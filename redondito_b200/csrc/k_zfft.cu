@@ -50,6 +50,8 @@ struct ZArgs {
   // the passes of the nonlinear step (Z_POT, Z_RHS, Z_DLADD)
   ZNlArgs nl;
   const double *z, *zinv;  // r, 1/r
+  bool digits;  // general lengths: the passes of fft_engine.cuh
+  int nbuf;     // their buffers: one where every radix is done in place
 };
 
 // modes that keep the whole input column (every row) beside the transform's
@@ -356,17 +358,27 @@ __global__ void __launch_bounds__(Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::THR
 // 528 columns at nz 58 (2 29) and 33 (3 11): 7.1 and 6.3 us, against 221 and
 // 42 us with one thread per butterfly in place and 32 columns per CTA; nz 90,
 // 14706 columns, plain: 19-27 against 52-59 us.
-template <int MODE, int IO>
-__global__ void __launch_bounds__(ZTHREADS, 2) zfft_gen_kernel(ZArgs a, int lg) {
+//
+// DIGITS: the decimation-in-frequency and -in-time passes of fft_engine.cuh
+// instead, the spectrum in digit-reversed order between them.  Mixed plans
+// take these on FP64 arrays: the fp32 steps after a z transform round, and a
+// forward continuation (weights up to 3.7e3) amplifies what a last-bit change
+// flips there, so another order of the FP64 sums moves their results by 3e-6.
+template <int MODE, int IO, bool DIGITS>
+__global__ void __launch_bounds__(ZTHREADS, DIGITS ? 4 : 2) zfft_gen_kernel(ZArgs a, int lg) {
   extern __shared__ double2 sm[];
   const int LB = 1 << lg, nz = a.nz, nlm = a.nlm, lm0 = blockIdx.x << lg, tid = threadIdx.x;
   const bool cont = MODE != Z_INV && a.C > 0;
   const int nload = cont ? a.N : nz, total = nz << lg;
   constexpr bool KEEP = zkeep(MODE);
-  double2* orig = sm + 2 * total;
+  double2* orig = sm + a.nbuf * total;
+  const int* __restrict__ rev = a.fd.rev;
+  // slot of frequency k
+  auto slot = [&](int k) { return DIGITS ? __ldg(rev + k) : k; };
   for (int idx = tid; idx < (KEEP ? total : nload << lg); idx += ZTHREADS) {
-    const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
-    zload<IO>(a, (KEEP ? orig : sm) + idx, (size_t)r * nlm + lm, lm < nlm);
+    const int r = idx >> lg, c = idx & (LB - 1), lm = lm0 + c;
+    const int to = MODE == Z_INV ? (slot(r) << lg) + c : idx;
+    zload<IO>(a, (KEEP ? orig : sm) + to, (size_t)r * nlm + lm, lm < nlm);
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -384,21 +396,28 @@ __global__ void __launch_bounds__(ZTHREADS, 2) zfft_gen_kernel(ZArgs a, int lg) 
     __syncthreads();
   }
   constexpr int SG = MODE == Z_INV ? 1 : -1;  // first transform's sign
-  double2* x = fg::run<SG>(sm, sm + total, nz, a.fd.gf, 0, a.fd.ng, lg, a.fd.tw);
+  const FftGeom g{nz, LB, 1, LB, 0, false};
+  double2* x;
+  if constexpr (!DIGITS) x = fg::run<SG>(sm, sm + total, nz, a.fd.gf, 0, a.fd.ng, lg, a.fd.tw);
+  else if constexpr (MODE == Z_INV) x = fft_dit2(sm, sm + total, a.fd, g, 1);
+  else x = fft_dif2(sm, sm + total, a.fd, g, -1);
   if constexpr (MODE != Z_FWD && MODE != Z_INV) {
     for (int idx = tid; idx < total; idx += ZTHREADS) {
-      const int k = idx >> lg;
-      const double2 v = div_nz(x[idx], nz);
-      x[idx] = MODE == Z_FILTER ? cscale(v, a.filt[k]) : cmul(a.kfac[k], v);
+      const int k = idx >> lg, o = (slot(k) << lg) + (idx & (LB - 1));
+      const double2 v = div_nz(x[o], nz);
+      x[o] = MODE == Z_FILTER ? cscale(v, a.filt[k]) : cmul(a.kfac[k], v);
     }
     __syncthreads();
-    x = fg::run<1>(x, x == sm ? sm + total : sm, nz, a.fd.gf, 0, a.fd.ng, lg, a.fd.tw);
+    double2* y = x == sm ? sm + total : sm;
+    if constexpr (DIGITS) x = fft_dit2(x, y, a.fd, g, 1);
+    else x = fg::run<1>(x, y, nz, a.fd.gf, 0, a.fd.ng, lg, a.fd.tw);
   }
   for (int idx = tid; idx < total; idx += ZTHREADS) {
-    const int r = idx >> lg, lm = lm0 + (idx & (LB - 1));
+    const int r = idx >> lg, c = idx & (LB - 1), lm = lm0 + c;
     if (lm >= nlm) continue;
     const size_t o = (size_t)r * nlm + lm;
-    if constexpr (MODE == Z_FWD || MODE == Z_INV) zstore<IO>(a, o, MODE == Z_FWD ? div_nz(x[idx], nz) : x[idx]);
+    if constexpr (MODE == Z_FWD) zstore<IO>(a, o, div_nz(x[(slot(r) << lg) + c], nz));
+    else if constexpr (MODE == Z_INV) zstore<IO>(a, o, x[idx]);
     else zspectral_store<MODE, IO>(a, r, lm, o, x[idx], KEEP ? orig[idx] : x[idx]);
   }
 }
@@ -413,22 +432,35 @@ int zgen_lb(int nz, int nlm) {
   return lb;
 }
 
-template <int MODE, int IO>
-int launch_gen(const ZArgs& a, cudaStream_t st) {
+template <int MODE, int IO, bool DIGITS>
+int launch_gen_as(const ZArgs& a, cudaStream_t st) {
   static DeviceOnce once;
   if (!once.run([] {
-        return cudaFuncSetAttribute(zfft_gen_kernel<MODE, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        return cudaFuncSetAttribute(zfft_gen_kernel<MODE, IO, DIGITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     200 * 1024) == cudaSuccess &&
-               cudaFuncSetAttribute(zfft_gen_kernel<MODE, IO>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    100) == cudaSuccess;
+               cudaFuncSetAttribute(zfft_gen_kernel<MODE, IO, DIGITS>,
+                                    cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
       }))
     return SPH_ECUDA;
   int lg = 0;
   while ((1 << lg) < a.LB) ++lg;
-  const size_t smem = ((size_t)a.nz << lg) * sizeof(double2) * (zkeep(MODE) ? 3 : 2);
-  zfft_gen_kernel<MODE, IO><<<(a.nlm + a.LB - 1) / a.LB, ZTHREADS, smem, st>>>(a, lg);
+  const size_t smem = ((size_t)a.nz << lg) * sizeof(double2) * (a.nbuf + zkeep(MODE));
+  zfft_gen_kernel<MODE, IO, DIGITS><<<(a.nlm + a.LB - 1) / a.LB, ZTHREADS, smem, st>>>(a, lg);
   SPH_LAUNCH_OK();
   return SPH_OK;
+}
+
+template <int MODE, int IO>
+int launch_gen(ZArgs a, cudaStream_t st) {
+  a.nbuf = 2;
+  if constexpr (IO == ZIO_DD)
+    if (a.digits) {
+      a.nbuf = 1;
+      for (int i = 0; i < a.fd.npass; ++i)
+        if (!fft_inplace_radix(a.fd.pass[i].R)) a.nbuf = 2;
+      return launch_gen_as<MODE, IO, true>(a, st);
+    }
+  return launch_gen_as<MODE, IO, false>(a, st);
 }
 
 template <int MODE, int R1, int R2, int IO>
@@ -565,6 +597,7 @@ int make_zargs(const sph_plan* p, int mode, const void* in, void* out, int order
   a.nl = {};
   a.z = p->d_z;
   a.zinv = p->zinv;
+  a.digits = p->precision == SPH_MIXED;
   return SPH_OK;
 }
 

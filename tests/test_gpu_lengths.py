@@ -74,3 +74,31 @@ def test_z_lengths(lmax, nz, cols):
         S.fc_filter(G, x, "r")
         check(rel_l2(x.cpu().numpy(), P.fc_filter(a, "r")), 1e-11, f"nz {nz} filter")
     G.close()
+
+
+# A mixed plan's radial transforms of FP64 arrays (the passes of
+# fft_engine.cuh, odd primes one output per thread): 31 (one prime pass),
+# 39 = 3 13, 58 = 2 29, 81 = 3^4 (one buffer), 90 = 2 9 5, 289 = 17 17
+@pytest.mark.parametrize("nz", [31, 39, 58, 81, 90, 289])
+@pytest.mark.parametrize("cols", [0, 2])
+def test_z_lengths_mixed(nz, cols):
+    from redondito_b200 import sphp as S
+    lmax, nlat, nphi = 7, 24, 48
+    C, d = (25, 5) if nz < 200 else (0, 0)
+    P = O.Plan(lmax, nz, nlat=nlat, nphi=nphi, C=C, d=d)
+    G = S.Plan(lmax, nz, nlat=nlat, nphi=nphi, Cz=C, oz=d, precision=S.SPH_MIXED)
+    S.set_tiles(G, z_cols=cols)
+    a = random_spec(P, np.random.default_rng(nz))
+    x = dev(a)
+    S.fftp1d_real_to_complex_z(G, x)
+    f = P.z_forward(a)
+    check(rel_l2(x.cpu().numpy(), f), TOL, f"nz {nz} forward")
+    x = dev(f)
+    S.fftp1d_complex_to_real_z(G, x)
+    check(rel_l2(x.cpu().numpy(), P.z_inverse(f)), TOL, f"nz {nz} inverse")
+    if C:
+        b = G.new_spec()
+        for order in (1, "dlr"):
+            (S.dlr(G, dev(a), b) if order == "dlr" else S.derivr(G, dev(a), b, order, "r"))
+            check_derivative(b.cpu().numpy(), P, a, order, f"nz {nz}")
+    G.close()
