@@ -167,7 +167,7 @@ static int upload(T** dst, const T* src, size_t n) {
 static std::vector<void*> table_ptrs(const sph_plan* p) {
   return {p->P, p->dP, p->mPs, p->wfold, p->wfull, p->d_dir, p->d_z, p->kfac, p->filt, p->zinv, p->zinv2, p->d_ell,
           p->d_mbase, p->twz, p->twphi, p->twzf, p->twphif, p->revz, p->revphi, p->twpz, p->twpphi, p->twpzf,
-          p->twpphif, p->tw4f, p->tw4d, p->tilesA, p->tilesA32, p->tilesS, p->tilesS32, p->d_bplanes, p->d_toff};
+          p->twpphif, p->tw4f, p->tw4d, p->tilesA, p->tilesA64, p->tilesS, p->tilesS32, p->d_bplanes, p->d_toff};
 }
 
 PlanTables::~PlanTables() {
@@ -354,8 +354,8 @@ extern "C" int sph_plan_create(sph_plan** out, int lmax, int nlat, int nphi, int
     t4.insert(t4.end(), t4b.begin(), t4b.end());
     t4f.insert(t4f.end(), t4fb.begin(), t4fb.end());
   }
-  auto tA = row_tiles(lmax, 64, true, n2);
-  auto tA32 = row_tiles(lmax, 32, true, n2);
+  auto tA = row_tiles(lmax, 128, true, n2);
+  auto tA64 = row_tiles(lmax, 64, true, n2);
   auto tS = row_tiles(lmax, 64, false, n2);
   auto tS32 = row_tiles(lmax, 32, false, n2);
   // heaviest synthesis tiles (small m: K = lmax+1-m) first
@@ -390,12 +390,12 @@ extern "C" int sph_plan_create(sph_plan** out, int lmax, int nlat, int nphi, int
   UP(p->tw4f, t4f);
   UP(p->tw4d, t4);
   UP(p->tilesA, tA);
-  UP(p->tilesA32, tA32);
+  UP(p->tilesA64, tA64);
   UP(p->tilesS, tS);
   UP(p->tilesS32, tS32);
   if (Cz > 0) UP(p->d_dir, p->dir);
   p->ntilesA = (int)tA.size();
-  p->ntilesA32 = (int)tA32.size();
+  p->ntilesA64 = (int)tA64.size();
   p->ntilesS = (int)tS.size();
   p->ntilesS32 = (int)tS32.size();
   p->fz.tw = p->twz;

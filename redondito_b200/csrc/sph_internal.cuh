@@ -120,10 +120,10 @@ struct sph_plan {
   int tw4off = 0;
   FftDesc fz, fphi;
   // Legendre work lists (device)
-  LegTile* tilesA = nullptr;   // analysis: (m, l0) blocks of 64 l
+  LegTile* tilesA = nullptr;   // analysis: (m, l0) blocks of 128 l
   int ntilesA = 0;
-  LegTile* tilesA32 = nullptr; // vector analysis: blocks of 32 l
-  int ntilesA32 = 0;
+  LegTile* tilesA64 = nullptr; // vector analysis: blocks of 64 l
+  int ntilesA64 = 0;
   LegTile* tilesS = nullptr;   // synthesis: (m, i0) blocks of 64 nodes
   int ntilesS = 0;
   LegTile* tilesS32 = nullptr; // vector synthesis: blocks of 32 nodes
