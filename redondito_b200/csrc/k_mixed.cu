@@ -1838,22 +1838,15 @@ int phi_pairs(const sph_plan* p) {
   return 1;
 }
 
-template <typename K>
-int run_phi(K kernel, const Phi32Args& a, dim3 grid, size_t smem, cudaStream_t st) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
-      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
+template <auto KERNEL>
+int run_phi(const Phi32Args& a, dim3 grid, int threads, size_t smem, cudaStream_t st) {
+  static DeviceOnce once;
+  if (!once.run([] {
+        return cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
+               cudaFuncSetAttribute(KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
+      }))
     return SPH_ECUDA;
-  kernel<<<grid, PTHREADS, smem, st>>>(a);
-  SPH_LAUNCH_OK();
-  return SPH_OK;
-}
-
-template <typename K>
-int run_phi4(K kernel, const Phi32Args& a, dim3 grid, int threads, size_t smem, cudaStream_t st) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
-    return SPH_ECUDA;
-  kernel<<<grid, threads, smem, st>>>(a);
+  KERNEL<<<grid, threads, smem, st>>>(a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -1862,7 +1855,8 @@ template <int N, int NP, bool FWD, typename GT>
 int phi4_np(const Phi32Args& a, dim3 grid, cudaStream_t st) {
   static_assert(FWD, "the four-step form is forward only");
   using C = P4<N, NP>;
-  return run_phi4(phi4_fwd32<N, NP, GT>, a, grid, C::THREADS, C::SMEM_FWD, st);
+  static_assert(C::SMEM_FWD <= 200 * 1024, "shared memory limit of run_phi");
+  return run_phi<phi4_fwd32<N, NP, GT>>(a, grid, C::THREADS, C::SMEM_FWD, st);
 }
 
 template <int N, bool FWD, typename GT>
@@ -1882,17 +1876,17 @@ int phi32_n(const Phi32Args& a, dim3 grid, size_t smem, cudaStream_t st) {
   switch (a.NP) {
     case 8:
       if constexpr (8 * N <= PMAXC)
-        return run_phi(FWD ? phi_fwd32<N, 8, GT> : phi_inv32<N, 8, GT>, a, grid, smem, st);
+        return run_phi<FWD ? phi_fwd32<N, 8, GT> : phi_inv32<N, 8, GT>>(a, grid, PTHREADS, smem, st);
       break;
     case 4:
       if constexpr (4 * N <= PMAXC)
-        return run_phi(FWD ? phi_fwd32<N, 4, GT> : phi_inv32<N, 4, GT>, a, grid, smem, st);
+        return run_phi<FWD ? phi_fwd32<N, 4, GT> : phi_inv32<N, 4, GT>>(a, grid, PTHREADS, smem, st);
       break;
     case 2:
       if constexpr (2 * N <= PMAXC)
-        return run_phi(FWD ? phi_fwd32<N, 2, GT> : phi_inv32<N, 2, GT>, a, grid, smem, st);
+        return run_phi<FWD ? phi_fwd32<N, 2, GT> : phi_inv32<N, 2, GT>>(a, grid, PTHREADS, smem, st);
       break;
-    case 1: return run_phi(FWD ? phi_fwd32<N, 1, GT> : phi_inv32<N, 1, GT>, a, grid, smem, st);
+    case 1: return run_phi<FWD ? phi_fwd32<N, 1, GT> : phi_inv32<N, 1, GT>>(a, grid, PTHREADS, smem, st);
   }
   return SPH_EINVAL;
 }
@@ -1957,7 +1951,7 @@ int phi3_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
     const long long ntiles = (long long)(p->nlat2 / NP) * p->nz * nfields;
     if (ntiles == 0) return SPH_OK;
     if (ntiles > (1ll << 30)) return PHI3_UNSUPPORTED;
-    int occ = 0;
+    static Residency residency;
     if constexpr (FWD) {
       Phi3Maps maps;
       if (!a.flag) return PHI3_UNSUPPORTED;
@@ -1971,19 +1965,15 @@ int phi3_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
       }
       for (int f = nfields; f < SPH_MAX_FIELDS; ++f) maps.lo[f] = maps.hi[f] = maps.lo[0];
       auto kern = phi3_fwd32<N, NP, GT>;
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-          cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, G::THREADS, smem) != cudaSuccess)
-        return SPH_ECUDA;
-      const int grid = (int)std::min<long long>(ntiles, (long long)std::max(1, occ) * std::max(1, p->nsm));
+      const int occ = residency.get(kern, G::THREADS, smem, PHI3_SMEM_MAX);
+      if (!occ) return SPH_ECUDA;
+      const int grid = (int)std::min<long long>(ntiles, (long long)occ * std::max(1, p->nsm));
       kern<<<grid, G::THREADS, smem, st>>>(a, (int)ntiles, maps);
     } else {
       auto kern = phi3_inv32<N, NP, GT>;
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-          cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, G::THREADS, smem) != cudaSuccess)
-        return SPH_ECUDA;
-      const int grid = (int)std::min<long long>(ntiles, (long long)std::max(1, occ) * std::max(1, p->nsm));
+      const int occ = residency.get(kern, G::THREADS, smem, PHI3_SMEM_MAX);
+      if (!occ) return SPH_ECUDA;
+      const int grid = (int)std::min<long long>(ntiles, (long long)occ * std::max(1, p->nsm));
       kern<<<grid, G::THREADS, smem, st>>>(a, (int)ntiles);
     }
     SPH_LAUNCH_OK();
@@ -2011,11 +2001,9 @@ int phi2_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
     constexpr int T = PHI2_T;
     const size_t smem = phi2_smem<N>();
     auto kb = phi2b_fwd32<N>;
-    int occ = 0;
-    if (cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(kb, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kb, T, smem) != cudaSuccess)
-      return SPH_ECUDA;
+    static Residency residency;
+    const int occ = residency.get(kb, T, smem, PHI3_SMEM_MAX);
+    if (!occ) return SPH_ECUDA;
     const int nq = p->nz * nfields, ngroups = p->nlat2 / PHI2_NP;
     for (int q0 = 0; q0 < nq; q0 += p->phi2_planes) {
       const int nb = std::min(p->phi2_planes, nq - q0);
@@ -2023,7 +2011,7 @@ int phi2_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
                                                                                                       q0);
       SPH_LAUNCH_OK();
       const int ntiles = nb * ngroups;
-      const int grid = std::min(ntiles, std::max(1, occ) * std::max(1, p->nsm));
+      const int grid = std::min(ntiles, occ * std::max(1, p->nsm));
       kb<<<grid, T, smem, st>>>(a, p->phi2, q0, nb, ntiles);
       SPH_LAUNCH_OK();
     }

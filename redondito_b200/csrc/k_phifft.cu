@@ -572,14 +572,13 @@ int phi3d_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
     if (ntiles == 0) return SPH_OK;
     if (ntiles > (1ll << 30)) return PHI3D_UNSUPPORTED;
     auto kern = phi3_inv64<N, NP>;
-    int occ = 0, dev = 0, nsm = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, G::THREADS, smem) != cudaSuccess ||
-        cudaGetDevice(&dev) != cudaSuccess ||
+    static Residency residency;
+    const int occ = residency.get(kern, G::THREADS, smem, G::SMEM_MAX);
+    int dev = 0, nsm = 0;
+    if (!occ || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return SPH_ECUDA;
-    const int grid = (int)std::min<long long>(ntiles, (long long)std::max(1, occ) * std::max(1, nsm));
+    const int grid = (int)std::min<long long>(ntiles, (long long)occ * std::max(1, nsm));
     kern<<<grid, G::THREADS, smem, st>>>(a, (int)ntiles);
     SPH_LAUNCH_OK();
     return SPH_OK;
@@ -855,9 +854,16 @@ int phi3c_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(CL);
-    int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) != cudaSuccess || nclusters < 1)
-      return PHI3C_UNSUPPORTED;
+    // clusters that fit the device, asked of the driver once per device
+    static std::atomic<int> fit[64];
+    int dev = 0, nclusters = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return SPH_ECUDA;
+    if (dev >= 0 && dev < 64) nclusters = fit[dev].load(std::memory_order_relaxed);
+    if (nclusters < 1) {
+      if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) != cudaSuccess || nclusters < 1)
+        return PHI3C_UNSUPPORTED;
+      if (dev >= 0 && dev < 64) fit[dev].store(nclusters, std::memory_order_relaxed);
+    }
     const long long ncl = std::min<long long>(nclusters, (ntiles + 0));
     cfg.gridDim = dim3((unsigned)(ncl * CL));
     if (cudaLaunchKernelEx(&cfg, kern, a, (int)ntiles, maps) != cudaSuccess) return SPH_ECUDA;
@@ -885,16 +891,19 @@ int pairs_per_cta(const sph_plan* p) {
   return 1;
 }
 
-template <typename K>
-bool smem_attr(K fn) {
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
-         cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
+template <auto KERNEL>
+bool smem_attr() {
+  static DeviceOnce once;
+  return once.run([] {
+    return cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) == cudaSuccess &&
+           cudaFuncSetAttribute(KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
+  });
 }
 
-template <typename K>
-int run(K kernel, const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
-  if (!smem_attr(kernel)) return SPH_ECUDA;
-  kernel<<<grid, PTHREADS, smem, st>>>(a);
+template <auto KERNEL>
+int run(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
+  if (!smem_attr<KERNEL>()) return SPH_ECUDA;
+  KERNEL<<<grid, PTHREADS, smem, st>>>(a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -903,10 +912,10 @@ template <int N>
 int launch_fwd_n(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
   if constexpr (N > 0) {
     switch (a.NP) {
-      case 8: if constexpr (8 * N <= PMAXC) return run(phi_fwd_ct<N, 8>, a, grid, smem, st); break;
-      case 4: if constexpr (4 * N <= PMAXC) return run(phi_fwd_ct<N, 4>, a, grid, smem, st); break;
-      case 2: if constexpr (2 * N <= PMAXC) return run(phi_fwd_ct<N, 2>, a, grid, smem, st); break;
-      case 1: return run(phi_fwd_ct<N, 1>, a, grid, smem, st);
+      case 8: if constexpr (8 * N <= PMAXC) return run<phi_fwd_ct<N, 8>>(a, grid, smem, st); break;
+      case 4: if constexpr (4 * N <= PMAXC) return run<phi_fwd_ct<N, 4>>(a, grid, smem, st); break;
+      case 2: if constexpr (2 * N <= PMAXC) return run<phi_fwd_ct<N, 2>>(a, grid, smem, st); break;
+      case 1: return run<phi_fwd_ct<N, 1>>(a, grid, smem, st);
     }
   }
   return SPH_EINVAL;
@@ -916,10 +925,10 @@ template <int N>
 int launch_inv_n(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
   if constexpr (N > 0) {
     switch (a.NP) {
-      case 8: if constexpr (8 * N <= PMAXC) return run(phi_inv_ct<N, 8>, a, grid, smem, st); break;
-      case 4: if constexpr (4 * N <= PMAXC) return run(phi_inv_ct<N, 4>, a, grid, smem, st); break;
-      case 2: if constexpr (2 * N <= PMAXC) return run(phi_inv_ct<N, 2>, a, grid, smem, st); break;
-      case 1: return run(phi_inv_ct<N, 1>, a, grid, smem, st);
+      case 8: if constexpr (8 * N <= PMAXC) return run<phi_inv_ct<N, 8>>(a, grid, smem, st); break;
+      case 4: if constexpr (4 * N <= PMAXC) return run<phi_inv_ct<N, 4>>(a, grid, smem, st); break;
+      case 2: if constexpr (2 * N <= PMAXC) return run<phi_inv_ct<N, 2>>(a, grid, smem, st); break;
+      case 1: return run<phi_inv_ct<N, 1>>(a, grid, smem, st);
     }
   }
   return SPH_EINVAL;
@@ -975,8 +984,8 @@ int launch_phi_fwd(const sph_plan* p, const double* const* grids, int nfields, c
   }
   int lg = 0, threads = 0;
   size_t gsmem = 0;
-  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run(phi_fwd_kernel, a, grid, smem, st);
-  if (!smem_attr(phi_fwd_gen)) return SPH_ECUDA;
+  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run<phi_fwd_kernel>(a, grid, smem, st);
+  if (!smem_attr<phi_fwd_gen>()) return SPH_ECUDA;
   grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
   phi_fwd_gen<<<grid, threads, gsmem, st>>>(a, lg);
   SPH_LAUNCH_OK();
@@ -1010,8 +1019,8 @@ int launch_phi_inv(const sph_plan* p, double* const* grids, int nfields, cudaStr
   }
   int lg = 0, threads = 0;
   size_t gsmem = 0;
-  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run(phi_inv_kernel, a, grid, smem, st);
-  if (!smem_attr(phi_inv_gen)) return SPH_ECUDA;
+  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run<phi_inv_kernel>(a, grid, smem, st);
+  if (!smem_attr<phi_inv_gen>()) return SPH_ECUDA;
   grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
   phi_inv_gen<<<grid, threads, gsmem, st>>>(a, lg);
   SPH_LAUNCH_OK();

@@ -180,7 +180,9 @@ def _check(fn, rc):
 
 
 def _call(name, *args):
-    _check(name, getattr(lib(), name)(*args))
+    rc = getattr(_lib or lib(), name)(*args)
+    if rc:
+        _check(name, rc)
 
 
 def nlat_for(lmax):
@@ -305,12 +307,12 @@ class Plan:
 
 
 def _ptr(t, shape, dtype):
-    if not isinstance(t, torch.Tensor) or t.device.type != "cuda":
+    if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise TypeError("fields must be CUDA tensors")
-    if t.dtype != dtype or tuple(t.shape) != tuple(shape) or not t.is_contiguous():
+    if t.dtype != dtype or t.shape != shape or not t.is_contiguous():
         raise ValueError(f"expected contiguous {dtype} tensor of shape {tuple(shape)}, "
                          f"got {t.dtype} {tuple(t.shape)}")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _g(plan, t):
@@ -355,8 +357,9 @@ def range_(n1, n2, nprocs, irank):
 
 
 def _stream(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 # ---------------------------------------------------------------- transforms
