@@ -629,12 +629,21 @@ struct P3c {
   static constexpr int SWB = ROWB >= 128 ? 3 : 2;               // swizzle: 2^SWB chunks of 16 bytes
   static constexpr int ITEMS_A = NPL * M, ITEMS_B = NPL * A * C, ITEMS_C = NPL * A * B;
   static constexpr int THREADS = ITEMS_A <= 64 ? 64 : (ITEMS_A + 31) / 32 * 32;
+  // step (C) and the fold in one from registers, on all warps but the first
+  // (four fields of 128 planes: nphi 1536 2.68 -> 2.55 ms, 768 606 -> 577 us;
+  // at nphi 384, where a third of the CTA would sit out step (C), 101 against
+  // 99 us)
+  static constexpr bool PAIRED = B == 16;
+  static constexpr int PAIRS = A / 2 * B;  // pairs of mirrored rows (ka, kb)
   static constexpr int PR = M | 1;
   static constexpr int SB = up_mod16(A * PR, 8 / NPL);
   static constexpr size_t XBYTES = (size_t)NPL * SB * sizeof(double2);
   static constexpr size_t TILE_BYTES = (size_t)2 * ROWS * ROWB;  // rings and mirrors
   static constexpr size_t STAGE = round_up(XBYTES > TILE_BYTES ? XBYTES : TILE_BYTES, 1024);
   static constexpr size_t SMEM = 2 * STAGE + (size_t)N * sizeof(double2) + 64;
+  // two CTAs per SM where shared memory allows and registers leave 128 a
+  // thread (nphi 768: 6 warps per SM were 897 us, 12 are 606)
+  static constexpr int MINB = 2 * (SMEM + 1024) <= 228 * 1024 && 2 * THREADS * 128 <= 65536 ? 2 : 1;
   // byte offset of staged element (row, column) within one half of a stage
   static __device__ __forceinline__ uint32_t off(int row, int col) {
     const uint32_t o = (uint32_t)(row * ROWB + col * 8);
@@ -659,7 +668,7 @@ struct GridMaps {
 };
 
 template <int N, int CL>
-__global__ void __launch_bounds__(P3c<N, CL>::THREADS, 1)
+__global__ void __launch_bounds__(P3c<N, CL>::THREADS, P3c<N, CL>::MINB)
     phi3c_fwd64(PhiArgs a, int ntiles, const __grid_constant__ GridMaps maps) {
   using G = P3c<N, CL>;
   constexpr int A = G::A, M = G::M, B = G::B, C = G::C, T = G::THREADS, NPL = G::NPL, NPC = G::NPC;
@@ -770,7 +779,7 @@ __global__ void __launch_bounds__(P3c<N, CL>::THREADS, 1)
       }
       __syncthreads();
     }
-    if constexpr (C > 1) {  // (C)
+    if constexpr (C > 1 && !G::PAIRED) {  // (C)
       for (int it = t; it < G::ITEMS_C; it += T) {
         const int ka = it % A, r2 = it / A, kb = r2 % B, bb = r2 / B;
         double2* row = X + bb * G::SB + ka * G::PR + C * kb;
@@ -783,25 +792,70 @@ __global__ void __launch_bounds__(P3c<N, CL>::THREADS, 1)
       }
       __syncthreads();
     }
-    // fold both parities of one (m, pair) from Z(m), Z(-m), as phi_fwd_ct;
-    // warp 0 takes no part: it holds no global stores at the releasing barrier
+    // the fold of both parities of one (m, pair) from Z(m), Z(-m), as
+    // phi_fwd_ct; warp 0 takes no part: it holds no global stores at the
+    // releasing barrier
     if (warp > 0) {
-      const int tf = t - 32;
       double2* Gp = a.G + (size_t)f * a.Gfield + (size_t)k * a.ldn + g * NPC + (int)rank * NPL + b;
       const size_t mstride = (size_t)2 * a.nz * a.ldn, pstride = (size_t)a.nz * a.ldn;
       const double W = __ldg(a.wfold + g * NPC + (int)rank * NPL + b);
-      auto zpos = [&](int m) {
-        const int q = m / A;
-        return (m % A) * G::PR + C * (q % B) + q / B;
-      };
-      for (int m = tf / NPL; m <= a.lmax; m += (T - 32) / NPL) {
-        const double2 Z = X[b * G::SB + zpos(m)];
-        const double2 Zc = X[b * G::SB + zpos(m == 0 ? 0 : N - m)];
+      const double2* Xb = X + b * G::SB;
+      auto emit = [&](int m, double2 Z, double2 Zc) {
+        if (m > a.lmax) return;
         // F(i) = (Z + conj Z(-m))/2, F(mirror) = -i (Z - conj Z(-m))/2
-        double2 Fi = make_double2(0.5 * (Z.x + Zc.x), 0.5 * (Z.y - Zc.y));
-        double2 Fm = make_double2(0.5 * (Z.y + Zc.y), -0.5 * (Z.x - Zc.x));
+        const double2 Fi = make_double2(0.5 * (Z.x + Zc.x), 0.5 * (Z.y - Zc.y));
+        const double2 Fm = make_double2(0.5 * (Z.y + Zc.y), -0.5 * (Z.x - Zc.x));
         Gp[m * mstride] = cscale(cadd(Fi, Fm), W);
         Gp[m * mstride + pstride] = cscale(csub(Fi, Fm), W);
+      };
+      if constexpr (!G::PAIRED) {
+        auto zpos = [&](int m) {
+          const int q = m / A;
+          return (m % A) * G::PR + C * (q % B) + q / B;
+        };
+        for (int m = (t - 32) / NPL; m <= a.lmax; m += (T - 32) / NPL)
+          emit(m, Xb[zpos(m)], Xb[zpos(m == 0 ? 0 : N - m)]);
+      } else {
+        // with step (C): the frequencies of the row (ka, kb) mirror, kc
+        // reversed, into one other row, so a thread transforms the two and
+        // folds from registers
+        auto load = [&](int ka, int kb, double2 (&u)[C]) {
+#pragma unroll
+          for (int c = 0; c < C; ++c) u[c] = Xb[ka * G::PR + C * kb + c];
+          ct::RD<double2, C, -1>::run(u);
+        };
+#pragma unroll 1
+        for (int j = (t - 32) / NPL; j < G::PAIRS; j += (T - 32) / NPL) {
+          // rows (ka, kb) and (A - ka, B - 1 - kb); in the places of ka = 0
+          // its rows kb and B - kb, then those of ka = A/2
+          const int sl = j / (A / 2);
+          int ka = j % (A / 2), kb = sl, kb2 = B - 1 - sl;
+          if (ka == 0 && sl < B / 2) {
+            kb2 = sl ? B - sl : B / 2;
+          } else if (ka == 0) {
+            ka = A / 2;
+            kb = sl - B / 2;
+            kb2 = B - 1 - kb;
+          }
+          double2 u[C], v[C];
+          load(ka, kb, u);
+          load(ka ? A - ka : 0, kb2, v);
+          if (ka == 0 && kb == 0) {  // two rows that mirror into themselves, the first kc into C - kc
+            emit(0, u[0], u[0]);
+#pragma unroll
+            for (int kc = 1; 2 * kc < C; ++kc) emit(A * B * kc, u[kc], u[C - kc]);
+#pragma unroll
+            for (int kc = 0; kc < C; ++kc)
+              if (2 * kc + 1 < C) emit(A * B * kc + A * B / 2, v[kc], v[C - 1 - kc]);
+          } else {
+#pragma unroll
+            for (int kc = 0; kc < C; ++kc) {
+              const int kk = ka + A * (kb + B * kc);
+              if (2 * kk < N) emit(kk, u[kc], v[C - 1 - kc]);
+              else emit(N - kk, v[C - 1 - kc], u[kc]);
+            }
+          }
+        }
       }
     }
     // this stage is refilled by TMA (async proxy) after the next barrier
