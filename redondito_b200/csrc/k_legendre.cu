@@ -140,6 +140,7 @@ static_assert(KZ * CP * 16 <= SMEM, "output staging");
 
 template <bool GROUP>
 __global__ void __launch_bounds__(128, 4) leg_analysis_kernel(LegArgs a0, LegGroup grp) {
+  grid_dependency_wait();
   using namespace an;
   extern __shared__ __align__(128) unsigned char sm[];
   LegArgs a;
@@ -263,6 +264,7 @@ constexpr int SMEM = STAGES * STAGE;
 
 template <bool GROUP>
 __global__ void __launch_bounds__(128, 4) leg_synthesis_kernel(LegArgs a0, LegGroup grp) {
+  grid_dependency_wait();
   using namespace sy;
   extern __shared__ __align__(128) unsigned char sm[];
   LegArgs a;
@@ -373,6 +375,7 @@ static_assert(2 * KZ * CP * 16 <= SMEM, "output staging");
 }  // namespace va
 
 __global__ void __launch_bounds__(256, 2) vec_analysis_kernel(LegArgs a) {
+  grid_dependency_wait();
   using namespace va;
   extern __shared__ __align__(128) unsigned char sm[];
   const int bx = blockIdx.x / a.nkb, by = blockIdx.x - bx * a.nkb;
@@ -500,6 +503,7 @@ constexpr int SMEM = STAGES * STAGE;
 }  // namespace vs
 
 __global__ void __launch_bounds__(256, 2) vec_synthesis_kernel(LegArgs a) {
+  grid_dependency_wait();
   using namespace vs;
   extern __shared__ __align__(128) unsigned char sm[];
   const int bx = blockIdx.x / a.nkb, by = blockIdx.x - bx * a.nkb;
@@ -628,7 +632,7 @@ int launch_leg_analysis(const sph_plan* p, int gfield, double2* spec, cudaStream
   static DeviceOnce once;
   if (!once.run([] { return set_smem(leg_analysis_kernel<false>, an::SMEM); })) return SPH_ECUDA;
   TimedLaunch tl(p, T_LEG_ANA, st);
-  leg_analysis_kernel<false><<<p->ntilesA * a.nkb, 128, an::SMEM, st>>>(a, LegGroup{});
+  launch_dependent(leg_analysis_kernel<false>, p->ntilesA * a.nkb, 128, an::SMEM, st, a, LegGroup{});
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -641,7 +645,7 @@ int launch_leg_synthesis(const sph_plan* p, const double2* spec, int gfield, cud
   static DeviceOnce once;
   if (!once.run([] { return set_smem(leg_synthesis_kernel<false>, sy::SMEM); })) return SPH_ECUDA;
   TimedLaunch tl(p, T_LEG_SYN, st);
-  leg_synthesis_kernel<false><<<p->ntilesS * a.nkb, 128, sy::SMEM, st>>>(a, LegGroup{});
+  launch_dependent(leg_synthesis_kernel<false>, p->ntilesS * a.nkb, 128, sy::SMEM, st, a, LegGroup{});
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -654,7 +658,7 @@ int launch_vec_analysis(const sph_plan* p, double2* s, double2* t, cudaStream_t 
   static DeviceOnce once;
   if (!once.run([] { return set_smem(vec_analysis_kernel, va::SMEM); })) return SPH_ECUDA;
   TimedLaunch tl(p, T_VEC_ANA, st);
-  vec_analysis_kernel<<<p->ntilesA64 * a.nkb, 256, va::SMEM, st>>>(a);
+  launch_dependent(vec_analysis_kernel, p->ntilesA64 * a.nkb, 256, va::SMEM, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -667,7 +671,7 @@ int launch_vec_synthesis(const sph_plan* p, const double2* s, const double2* t, 
   static DeviceOnce once;
   if (!once.run([] { return set_smem(vec_synthesis_kernel, vs::SMEM); })) return SPH_ECUDA;
   TimedLaunch tl(p, T_VEC_SYN, st);
-  vec_synthesis_kernel<<<p->ntilesS32 * a.nkb, 256, vs::SMEM, st>>>(a);
+  launch_dependent(vec_synthesis_kernel, p->ntilesS32 * a.nkb, 256, vs::SMEM, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -713,11 +717,11 @@ int leg_group_launch(const GroupLaunch& g, cudaStream_t st) {
   if (g.analysis) {
     static DeviceOnce once;
     if (!once.run([] { return set_smem(leg_analysis_kernel<true>, an::SMEM); })) return SPH_ECUDA;
-    leg_analysis_kernel<true><<<g.grid, 128, an::SMEM, st>>>(LegArgs{}, grp);
+    launch_dependent(leg_analysis_kernel<true>, g.grid, 128, an::SMEM, st, LegArgs{}, grp);
   } else {
     static DeviceOnce once;
     if (!once.run([] { return set_smem(leg_synthesis_kernel<true>, sy::SMEM); })) return SPH_ECUDA;
-    leg_synthesis_kernel<true><<<g.grid, 128, sy::SMEM, st>>>(LegArgs{}, grp);
+    launch_dependent(leg_synthesis_kernel<true>, g.grid, 128, sy::SMEM, st, LegArgs{}, grp);
   }
   SPH_LAUNCH_OK();
   return SPH_OK;

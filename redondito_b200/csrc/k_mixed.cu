@@ -251,6 +251,7 @@ struct TileCur {
 // ---------------------------------------------------------------- tensor-core kernel
 template <int MODE, bool G>
 __global__ void __launch_bounds__(TC_THREADS, 1) tc_gemm(TcLaunch L) {
+  grid_dependency_wait();
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
   uint64_t* full = bars;                 // [STAGES] data + table tiles landed
@@ -601,6 +602,7 @@ struct P4 {
 // row chunks of the analysis tiles.
 template <int N, int NP, typename GT>
 __global__ void __launch_bounds__(P4<N, NP>::THREADS, 2) phi4_fwd32(Phi32Args a) {
+  grid_dependency_wait();
   using C = P4<N, NP>;
   constexpr int N1 = C::N1, N2 = C::N2;
   extern __shared__ float2 sx[];
@@ -676,6 +678,7 @@ __global__ void __launch_bounds__(P4<N, NP>::THREADS, 2) phi4_fwd32(Phi32Args a)
 // chunks of the analysis tiles.
 template <int N, int NP, typename GT>
 __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd32(Phi32Args a) {
+  grid_dependency_wait();
   extern __shared__ float2 sf[];
   constexpr int Q = 2 * NP, JSTEP = PTHREADS / Q;
   const int nlat = a.nlat;
@@ -739,6 +742,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd32(Phi32Args a) {
 
 template <int N, int NP, typename GT>
 __global__ void __launch_bounds__(PTHREADS, 2) phi_inv32(Phi32Args a) {
+  grid_dependency_wait();
   extern __shared__ float2 sf[];
   constexpr int Q = 2 * NP, JSTEP = PTHREADS / Q;
   const int nlat = a.nlat;
@@ -850,6 +854,7 @@ __host__ __device__ constexpr int phi3_box_rows() {
 template <int N, int NP, typename GT>
 __global__ void __launch_bounds__(P3<N, NP>::THREADS, P3<N, NP>::MINB)
     phi3_fwd32(Phi32Args a, int ntiles, const __grid_constant__ Phi3Maps maps) {
+  grid_dependency_wait();
   using G = P3<N, NP>;
   constexpr int A = G::A, M = G::M, B = G::B, C = G::C, T = G::THREADS, BR = phi3_box_rows<N>();
   static_assert(N % BR == 0 && G::ONE_PASS, "box rows, single-pass geometry");
@@ -985,6 +990,7 @@ __global__ void __launch_bounds__(P3<N, NP>::THREADS, P3<N, NP>::MINB)
 
 template <int N, int NP, typename GT>
 __global__ void __launch_bounds__(P3<N, NP>::THREADS, P3<N, NP>::MINB_INV) phi3_inv32(Phi32Args a, int ntiles) {
+  grid_dependency_wait();
   using G = P3<N, NP>;
   constexpr int A = G::A, M = G::M, B = G::B, C = G::C, T = G::THREADS;
   static_assert(G::ONE_PASS, "single-pass geometry");
@@ -1094,6 +1100,7 @@ constexpr int PHI2_PB = 16, PHI2_NMC = 16, PHI2_NP = 8, PHI2_BATCH = 64;
 
 template <int N, typename GT>
 __global__ void __launch_bounds__(PHI2_PB* PHI2_NMC, 2) phi2a_fwd32(Phi32Args a, float2* img, int q0) {
+  grid_dependency_wait();
   using G = P3<N, PHI2_NP>;
   constexpr int A = G::A, M = G::M, PB = PHI2_PB, NMC = PHI2_NMC, SPB = A * NMC + 1;
   static_assert(M % NMC == 0, "nm chunks");
@@ -1134,6 +1141,7 @@ __host__ __device__ constexpr size_t phi2_smem() {
 
 template <int N>
 __global__ void __launch_bounds__(PHI2_T, 2) phi2b_fwd32(Phi32Args a, const float2* img, int q0, int nq, int ntiles) {
+  grid_dependency_wait();
   using G = P3<N, PHI2_NP>;
   constexpr int NP = PHI2_NP, A = G::A, M = G::M, B = G::B, C = G::C, T = PHI2_T;
   constexpr int XF = NP * G::SB;  // float2 per tile image
@@ -1238,6 +1246,7 @@ __global__ void __launch_bounds__(PHI2_T, 2) phi2b_fwd32(Phi32Args a, const floa
 template <typename GT>
 __global__ void cont_phys_kernel(const GT* __restrict__ f0, const GT* __restrict__ f1, const GT* __restrict__ f2,
                                  GT* out, const double* __restrict__ dir, int C, int d, int N, size_t npts) {
+  grid_dependency_wait();
   const int f = blockIdx.y;
   const GT* in = f == 0 ? f0 : (f == 1 ? f1 : f2);
   GT* o = out + (size_t)f * C * npts;
@@ -1265,6 +1274,7 @@ template <int D, typename GT>
 __global__ void __launch_bounds__(256) cont_phys_d(const GT* __restrict__ f0, const GT* __restrict__ f1,
                                                    const GT* __restrict__ f2, GT* out,
                                                    const double* __restrict__ dir, int C, int N, size_t npts) {
+  grid_dependency_wait();
   extern __shared__ double sdir[];  // dir(ii, jj) at ii + C jj
   for (int i = threadIdx.x; i < C * D; i += blockDim.x) sdir[i] = __ldg(dir + i);
   __syncthreads();
@@ -1304,6 +1314,7 @@ __global__ void __launch_bounds__(256) cont_phys_d(const GT* __restrict__ f0, co
 __global__ void spec_to_tiles(const double2* __restrict__ in, const double2* __restrict__ in2,
                               __nv_bfloat16* tiles, size_t tfield, const long long* __restrict__ toff,
                               const int* __restrict__ mbase, int lmax, int nlm) {
+  grid_dependency_wait();
   const int m = blockIdx.x, k = blockIdx.y, f = blockIdx.z;
   const double2* src = (f ? in2 : in) + (size_t)k * nlm + mbase[m] - m;
   __nv_bfloat16* T = tiles + (size_t)f * tfield;
@@ -1372,6 +1383,7 @@ __device__ __forceinline__ void cp_async16zf(void* dst, const void* src, int src
 // (its 16-point steps spill heavily at 80)
 template <int NZ, typename TI, bool DER = false>
 __global__ void __launch_bounds__(ZT_THREADS, (DER && NZ >= 256) ? 2 : 3) zinv_tiles(ZtArgs a) {
+  grid_dependency_wait();
   extern __shared__ double2 zs[];  // element e of column j at j + ZT_PITCH e
   const int2 it = a.items[blockIdx.x];
   const int m = it.x, c = it.y, t = threadIdx.x;
@@ -1826,7 +1838,7 @@ int run_tc(const sph_plan* p, const TcSet& set, TcArgs a, cudaStream_t st) {
   L.total = (int)nunits;
   L.flag = p->dflag;
   const int grid = (int)std::min<long long>(nunits, std::max(1, p->nsm));
-  tc_gemm<MODE, false><<<grid, TC_THREADS, TC_SMEM, st>>>(L);
+  launch_dependent(tc_gemm<MODE, false>, grid, TC_THREADS, TC_SMEM, st, L);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -1846,7 +1858,7 @@ int run_phi(const Phi32Args& a, dim3 grid, int threads, size_t smem, cudaStream_
                cudaFuncSetAttribute(KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout, 100) == cudaSuccess;
       }))
     return SPH_ECUDA;
-  KERNEL<<<grid, threads, smem, st>>>(a);
+  launch_dependent(KERNEL, grid, threads, smem, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -1968,13 +1980,13 @@ int phi3_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
       const int occ = residency.get(kern, G::THREADS, smem, PHI3_SMEM_MAX);
       if (!occ) return SPH_ECUDA;
       const int grid = (int)std::min<long long>(ntiles, (long long)occ * std::max(1, p->nsm));
-      kern<<<grid, G::THREADS, smem, st>>>(a, (int)ntiles, maps);
+      launch_dependent(kern, grid, G::THREADS, smem, st, a, (int)ntiles, maps);
     } else {
       auto kern = phi3_inv32<N, NP, GT>;
       const int occ = residency.get(kern, G::THREADS, smem, PHI3_SMEM_MAX);
       if (!occ) return SPH_ECUDA;
       const int grid = (int)std::min<long long>(ntiles, (long long)occ * std::max(1, p->nsm));
-      kern<<<grid, G::THREADS, smem, st>>>(a, (int)ntiles);
+      launch_dependent(kern, grid, G::THREADS, smem, st, a, (int)ntiles);
     }
     SPH_LAUNCH_OK();
     return SPH_OK;
@@ -2007,12 +2019,12 @@ int phi2_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
     const int nq = p->nz * nfields, ngroups = p->nlat2 / PHI2_NP;
     for (int q0 = 0; q0 < nq; q0 += p->phi2_planes) {
       const int nb = std::min(p->phi2_planes, nq - q0);
-      phi2a_fwd32<N, GT><<<dim3(p->nlat2 / PHI2_PB, G::M / PHI2_NMC, nb), PHI2_PB * PHI2_NMC, 0, st>>>(a, p->phi2,
+      launch_dependent(phi2a_fwd32<N, GT>, dim3(p->nlat2 / PHI2_PB, G::M / PHI2_NMC, nb), PHI2_PB * PHI2_NMC, 0, st, a, p->phi2,
                                                                                                       q0);
       SPH_LAUNCH_OK();
       const int ntiles = nb * ngroups;
       const int grid = std::min(ntiles, occ * std::max(1, p->nsm));
-      kb<<<grid, T, smem, st>>>(a, p->phi2, q0, nb, ntiles);
+      launch_dependent(kb, grid, T, smem, st, a, p->phi2, q0, nb, ntiles);
       SPH_LAUNCH_OK();
     }
     return SPH_OK;
@@ -2115,13 +2127,13 @@ int cont_phys_t(const sph_plan* p, const void* const* grids, int nfields, cudaSt
   switch (p->d) {
 #define CASE(D)                                                                                               \
   case D:                                                                                                     \
-    cont_phys_d<D, GT><<<dim3(blocks, nfields), 256, smem, st>>>(f[0], f[1], f[2], out, p->d_dir, p->C, p->N, \
+    launch_dependent(cont_phys_d<D, GT>, dim3(blocks, nfields), 256, smem, st, f[0], f[1], f[2], out, p->d_dir, p->C, p->N, \
                                                                   npts);                                     \
     break;
     CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7) CASE(8)
 #undef CASE
     default:
-      cont_phys_kernel<GT><<<dim3(blocks, nfields), 256, 0, st>>>(f[0], f[1], f[2], out, p->d_dir, p->C, p->d,
+      launch_dependent(cont_phys_kernel<GT>, dim3(blocks, nfields), 256, 0, st, f[0], f[1], f[2], out, p->d_dir, p->C, p->d,
                                                                   p->N, npts);
   }
   SPH_LAUNCH_OK();
@@ -2222,7 +2234,7 @@ int launch_tc_synthesis(const sph_plan* p, int vector, const double2* in, const 
   a.tiles = reinterpret_cast<const __nv_bfloat16*>(p->Tsyn);
   {
     TimedLaunch tl(p, T_OPS, st);
-    spec_to_tiles<<<dim3(p->lmax + 1, p->nz, vector ? 2 : 1), 32, 0, st>>>(
+    launch_dependent(spec_to_tiles, dim3(p->lmax + 1, p->nz, vector ? 2 : 1), 32, 0, st, 
         in, in2, reinterpret_cast<__nv_bfloat16*>(p->Tsyn), p->Tsynfield, p->d_toff, p->d_mbase, p->lmax, p->nlm);
     SPH_LAUNCH_OK();
   }
@@ -2280,10 +2292,10 @@ int tc_group_launch(const GroupLaunch& g, int* flag, cudaStream_t st) {
   L.flag = flag;
   if (g.analysis) {
     if (!tc_attr<ANA_S, true>()) return SPH_ECUDA;
-    tc_gemm<ANA_S, true><<<g.grid, TC_THREADS, TC_SMEM, st>>>(L);
+    launch_dependent(tc_gemm<ANA_S, true>, g.grid, TC_THREADS, TC_SMEM, st, L);
   } else {
     if (!tc_attr<SYN_S, true>()) return SPH_ECUDA;
-    tc_gemm<SYN_S, true><<<g.grid, TC_THREADS, TC_SMEM, st>>>(L);
+    launch_dependent(tc_gemm<SYN_S, true>, g.grid, TC_THREADS, TC_SMEM, st, L);
   }
   SPH_LAUNCH_OK();
   return SPH_OK;
@@ -2313,7 +2325,7 @@ int zinv_tiles_run(const sph_plan* p, const ZtArgs& a, cudaStream_t st) {
                                     100) == cudaSuccess;
       }))
     return SPH_ECUDA;
-  zinv_tiles<NZ, TI, DER><<<p->nztitems, ZT_THREADS, smem, st>>>(a);
+  launch_dependent(zinv_tiles<NZ, TI, DER>, p->nztitems, ZT_THREADS, smem, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -2382,7 +2394,7 @@ int launch_tc_synthesis_tiles(const sph_plan* p, int vector, cudaStream_t st) {
 
 int launch_spec_to_tiles_field(const sph_plan* p, const double2* in, int field, cudaStream_t st) {
   if (p->precision != SPH_MIXED || field < 0 || field >= SPH_MAX_FIELDS) return SPH_EINVAL;
-  spec_to_tiles<<<dim3(p->lmax + 1, p->nz, 1), 32, 0, st>>>(
+  launch_dependent(spec_to_tiles, dim3(p->lmax + 1, p->nz, 1), 32, 0, st, 
       in, nullptr, reinterpret_cast<__nv_bfloat16*>(p->Tsyn) + (size_t)field * p->Tsynfield, p->Tsynfield,
       p->d_toff, p->d_mbase, p->lmax, p->nlm);
   SPH_LAUNCH_OK();

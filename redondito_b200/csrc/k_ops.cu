@@ -19,12 +19,14 @@ int ew_blocks(size_t n) {
 // derivr_k (src/pseudo/pseudospec_hd.f90:60-98): b = (i kz)^p a
 __global__ void kmul_kernel(const double2* __restrict__ a, double2* __restrict__ b,
                             const double2* __restrict__ f, int nlm, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
     b[q] = cmul(f[q / nlm], a[q]);
 }
 
 // fc_filter_k (pseudospec_hd.f90:407-440)
 __global__ void rowscale_kernel(double2* a, const double* __restrict__ f, int nlm, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
     a[q] = cscale(a[q], f[q / nlm]);
 }
@@ -32,6 +34,7 @@ __global__ void rowscale_kernel(double2* a, const double* __restrict__ f, int nl
 // laplang (pseudospec_hd.f90:138-172): b = -l(l+1) a
 __global__ void laplang_kernel(const double2* __restrict__ a, double2* __restrict__ b,
                                const int* __restrict__ ell, int nlm, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     int l = ell[q % nlm];
     b[q] = cscale(a[q], (double)(-l * (l + 1)));
@@ -41,6 +44,7 @@ __global__ void laplang_kernel(const double2* __restrict__ a, double2* __restric
 // multr (pseudospec_hd.f90:175-208): b = z^p a, integer p as Fortran's z**p
 __global__ void multr_kernel(const double2* __restrict__ a, double2* __restrict__ b,
                              const double* __restrict__ z, int power, int nlm, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     double zk = z[q / nlm], zp = 1.0;
     int ap = power < 0 ? -power : power;
@@ -52,6 +56,7 @@ __global__ void multr_kernel(const double2* __restrict__ a, double2* __restrict_
 
 // saxpby_c / saxpby_r (pseudospec_hd.f90:291-366): z = a x + b y
 __global__ void saxpby_kernel(double* z, const double* x, double a, const double* y, double b, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
     z[q] = a * x[q] + b * y[q];
 }
@@ -61,6 +66,7 @@ __global__ void prodvec_kernel(const double* __restrict__ ar, const double* __re
                                const double* __restrict__ ap, const double* __restrict__ br,
                                const double* __restrict__ bt, const double* __restrict__ bp,
                                double* cr, double* ct, double* cp, size_t nphys, size_t ntot) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < ntot; q += (size_t)gridDim.x * blockDim.x) {
     if (q < nphys) {
       double xr = ar[q], xt = at[q], xp = ap[q], yr = br[q], yt = bt[q], yp = bp[q];
@@ -77,6 +83,7 @@ __global__ void prodvec_kernel(const double* __restrict__ ar, const double* __re
 
 // dirichlet (src/boundary/boundary_mod.f90:62-93): rows 1 and N
 __global__ void dirichlet_kernel(double2* a, int nlm, int N) {
+  grid_dependency_wait();
   for (int lm = blockIdx.x * blockDim.x + threadIdx.x; lm < nlm; lm += gridDim.x * blockDim.x) {
     a[lm] = make_double2(0.0, 0.0);
     a[(size_t)(N - 1) * nlm + lm] = make_double2(0.0, 0.0);
@@ -105,6 +112,7 @@ __device__ __forceinline__ double2 reconstruct_col(const double2* f, int lm, int
 
 __global__ void reconstruct_kernel(double2* f, const double* __restrict__ neu, const double* __restrict__ a,
                                    int nlm, int N, int d, int boun, int robin) {
+  grid_dependency_wait();
   for (int lm = blockIdx.x * blockDim.x + threadIdx.x; lm < nlm; lm += gridDim.x * blockDim.x) {
     const int b = boun == 0 ? 0 : N - 1;
     const double2 g = f[(size_t)b * nlm + lm];
@@ -117,6 +125,7 @@ __global__ void reconstruct_kernel(double2* f, const double* __restrict__ neu, c
 // -2/rext outside (outward normal derivatives)
 __global__ void bc_walls_kernel(double2* tor, const double* __restrict__ neu, int nlm, int N, int d, int kin,
                                 int kout, double ain, double aout) {
+  grid_dependency_wait();
   for (int lm = blockIdx.x * blockDim.x + threadIdx.x; lm < nlm; lm += gridDim.x * blockDim.x) {
     for (int w = 0; w < 2; ++w) {
       const int b = w == 0 ? 0 : N - 1;
@@ -150,6 +159,7 @@ __global__ void __launch_bounds__(256, 2) invdl_kernel(const double2* __restrict
                                                        const double* __restrict__ binv,
                                                        const int* __restrict__ mbase, int lm0, int nlm, int N,
                                                        int nz) {
+  grid_dependency_wait();
   extern __shared__ double Ph[];  // [K rounded up to 16][IDL_LD]
   const int l = gridDim.x - blockIdx.x;  // the l with most modes first
   const int m0 = blockIdx.y * IDL_M;
@@ -229,6 +239,7 @@ __global__ void __launch_bounds__(256, 2) invdl_kernel(const double2* __restrict
 __global__ void bc_fast_kernel(double2* phi, const double2* __restrict__ w, const double* __restrict__ d2bor,
                                const int* __restrict__ ell, const double* __restrict__ z, int nlm, int nz,
                                int N) {
+  grid_dependency_wait();
   for (int lm = blockIdx.x * blockDim.x + threadIdx.x; lm < nlm; lm += gridDim.x * blockDim.x) {
     int l = ell[lm];
     if (l == 0) {
@@ -259,6 +270,7 @@ __global__ void bc_fast_kernel(double2* phi, const double2* __restrict__ w, cons
 // the toroidal potential of curl u: b = -a / r
 __global__ void neg_over_r_kernel(const double2* __restrict__ a, double2* __restrict__ b,
                                   const double* __restrict__ zinv, int nlm) {
+  grid_dependency_wait();
   const double f = -zinv[blockIdx.y];
   const size_t row = (size_t)blockIdx.y * nlm;
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nlm; q += gridDim.x * blockDim.x)
@@ -273,6 +285,7 @@ __global__ void __launch_bounds__(EW_THREADS)
                           const double* __restrict__ br, const double* __restrict__ bt, const double* __restrict__ bp,
                           double* cr, double* ct, double* cp, const double* __restrict__ w,
                           const double* __restrict__ z, int nlat, int nphi, int N, double scale, double* acc) {
+  grid_dependency_wait();
   __shared__ double red[EW_THREADS / 32];
   const int half = nlat / 2, n = half * nphi;  // pairs of nodes of one plane
   const size_t plane = (size_t)n * blockIdx.y;
@@ -309,7 +322,7 @@ int launch_kmul(const sph_plan* p, const double2* a, double2* b, int order, cuda
     return SPH_OK;
   }
   TimedLaunch tl(p, T_OPS, st);
-  kmul_kernel<<<ew_blocks(n), EW_THREADS, 0, st>>>(a, b, p->kfac + (size_t)(order - 1) * p->nz, p->nlmv, n);
+  launch_dependent(kmul_kernel, ew_blocks(n), EW_THREADS, 0, st, a, b, p->kfac + (size_t)(order - 1) * p->nz, p->nlmv, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -317,7 +330,7 @@ int launch_kmul(const sph_plan* p, const double2* a, double2* b, int order, cuda
 int launch_filter_k(const sph_plan* p, double2* a, cudaStream_t st) {
   size_t n = spec_view(p);
   TimedLaunch tl(p, T_OPS, st);
-  rowscale_kernel<<<ew_blocks(n), EW_THREADS, 0, st>>>(a, p->filt, p->nlmv, n);
+  launch_dependent(rowscale_kernel, ew_blocks(n), EW_THREADS, 0, st, a, p->filt, p->nlmv, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -325,7 +338,7 @@ int launch_filter_k(const sph_plan* p, double2* a, cudaStream_t st) {
 int launch_laplang(const sph_plan* p, const double2* a, double2* b, cudaStream_t st) {
   size_t n = spec_view(p);
   TimedLaunch tl(p, T_OPS, st);
-  laplang_kernel<<<ew_blocks(n), EW_THREADS, 0, st>>>(a, b, p->d_ell + p->lm0, p->nlmv, n);
+  launch_dependent(laplang_kernel, ew_blocks(n), EW_THREADS, 0, st, a, b, p->d_ell + p->lm0, p->nlmv, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -333,7 +346,7 @@ int launch_laplang(const sph_plan* p, const double2* a, double2* b, cudaStream_t
 int launch_multr(const sph_plan* p, const double2* a, double2* b, int power, cudaStream_t st) {
   size_t n = spec_view(p);
   TimedLaunch tl(p, T_OPS, st);
-  multr_kernel<<<ew_blocks(n), EW_THREADS, 0, st>>>(a, b, p->d_z, power, p->nlmv, n);
+  launch_dependent(multr_kernel, ew_blocks(n), EW_THREADS, 0, st, a, b, p->d_z, power, p->nlmv, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -341,7 +354,7 @@ int launch_multr(const sph_plan* p, const double2* a, double2* b, int power, cud
 int launch_saxpby(const sph_plan* p, double* z, const double* x, double a, const double* y, double b,
                   size_t n, cudaStream_t st) {
   TimedLaunch tl(p, T_OPS, st);
-  saxpby_kernel<<<ew_blocks(n), EW_THREADS, 0, st>>>(z, x, a, y, b, n);
+  launch_dependent(saxpby_kernel, ew_blocks(n), EW_THREADS, 0, st, z, x, a, y, b, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -353,7 +366,7 @@ int launch_prodvec(const sph_plan* p, const double* const* A, const double* cons
   const int nphys_planes = std::max(0, std::min(p->nzv, p->N - p->k0));
   size_t ntot = plane * p->nzv, nphys = plane * nphys_planes;
   TimedLaunch tl(p, T_OPS, st);
-  prodvec_kernel<<<ew_blocks(ntot), EW_THREADS, 0, st>>>(A[0], A[1], A[2], B[0], B[1], B[2], Cout[0],
+  launch_dependent(prodvec_kernel, ew_blocks(ntot), EW_THREADS, 0, st, A[0], A[1], A[2], B[0], B[1], B[2], Cout[0],
                                                         Cout[1], Cout[2], nphys, ntot);
   SPH_LAUNCH_OK();
   return SPH_OK;
@@ -361,7 +374,7 @@ int launch_prodvec(const sph_plan* p, const double* const* A, const double* cons
 
 int launch_dirichlet(const sph_plan* p, double2* a, cudaStream_t st) {
   TimedLaunch tl(p, T_OPS, st);
-  dirichlet_kernel<<<ew_blocks(p->nlmv), EW_THREADS, 0, st>>>(a, p->nlmv, p->N);
+  launch_dependent(dirichlet_kernel, ew_blocks(p->nlmv), EW_THREADS, 0, st, a, p->nlmv, p->N);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -369,7 +382,7 @@ int launch_dirichlet(const sph_plan* p, double2* a, cudaStream_t st) {
 int launch_bc_walls(const sph_plan* p, double2* tor, cudaStream_t st) {
   if ((p->bck[0] || p->bck[1]) && (!p->d_neu || p->neu[0].empty())) return SPH_ENOTREADY;
   TimedLaunch tl(p, T_OPS, st);
-  bc_walls_kernel<<<ew_blocks(p->nlmv), EW_THREADS, 0, st>>>(tor, p->d_neu, p->nlmv, p->N, p->d, p->bck[0],
+  launch_dependent(bc_walls_kernel, ew_blocks(p->nlmv), EW_THREADS, 0, st, tor, p->d_neu, p->nlmv, p->N, p->d, p->bck[0],
                                                              p->bck[1], 2.0 / p->z[0], -2.0 / p->z[p->N - 1]);
   SPH_LAUNCH_OK();
   return SPH_OK;
@@ -379,7 +392,7 @@ int launch_reconstruct(const sph_plan* p, double2* f, int boun, int ord, const d
   if ((boun != 0 && boun != 1) || (ord != 1 && ord != 2)) return SPH_EINVAL;
   if (!p->d_neu || p->neu[ord - 1].empty() || p->N < p->d) return SPH_ENOTREADY;
   TimedLaunch tl(p, T_OPS, st);
-  reconstruct_kernel<<<ew_blocks(p->nlmv), EW_THREADS, 0, st>>>(f, p->d_neu + (size_t)(ord - 1) * p->d, a, p->nlmv,
+  launch_dependent(reconstruct_kernel, ew_blocks(p->nlmv), EW_THREADS, 0, st, f, p->d_neu + (size_t)(ord - 1) * p->d, a, p->nlmv,
                                                                p->N, p->d, boun, a != nullptr);
   SPH_LAUNCH_OK();
   return SPH_OK;
@@ -400,14 +413,14 @@ int launch_invDl(const sph_plan* p, const double2* phi, double2* w, cudaStream_t
     return SPH_ECUDA;
   dim3 grid(p->lmax, (p->lmax + 1 + IDL_M - 1) / IDL_M);
   TimedLaunch tl(p, T_OPS, st);
-  invdl_kernel<<<grid, 256, smem, st>>>(phi, w, p->binv, p->d_mbase, p->lm0, p->nlmv, p->N, p->nz);
+  launch_dependent(invdl_kernel, grid, 256, smem, st, phi, w, p->binv, p->d_mbase, p->lm0, p->nlmv, p->N, p->nz);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
 
 int launch_bc_fast_rows(const sph_plan* p, double2* phi, const double2* w, cudaStream_t st) {
   TimedLaunch tl(p, T_OPS, st);
-  bc_fast_kernel<<<ew_blocks(p->nlmv), EW_THREADS, 0, st>>>(phi, w, p->d2bor, p->d_ell + p->lm0, p->d_z, p->nlmv,
+  launch_dependent(bc_fast_kernel, ew_blocks(p->nlmv), EW_THREADS, 0, st, phi, w, p->d2bor, p->d_ell + p->lm0, p->d_z, p->nlmv,
                                                             p->nz, p->N);
   SPH_LAUNCH_OK();
   return SPH_OK;
@@ -416,7 +429,7 @@ int launch_bc_fast_rows(const sph_plan* p, double2* phi, const double2* w, cudaS
 int launch_neg_over_r(const sph_plan* p, const double2* in, double2* out, cudaStream_t st) {
   TimedLaunch tl(p, T_OPS, st);
   const dim3 grid(std::min((p->nlm + EW_THREADS - 1) / EW_THREADS, 64), p->nz);
-  neg_over_r_kernel<<<grid, EW_THREADS, 0, st>>>(in, out, p->zinv, p->nlm);
+  launch_dependent(neg_over_r_kernel, grid, EW_THREADS, 0, st, in, out, p->zinv, p->nlm);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -427,7 +440,7 @@ int launch_prodvec_energy(const sph_plan* p, double* const* A, double* const* B,
   const int n = p->nlat / 2 * p->nphi;
   TimedLaunch tl(p, T_OPS, st);
   const dim3 grid(std::max(1, std::min((n + EW_THREADS - 1) / EW_THREADS, 32)), p->N);
-  prodvec_energy_kernel<<<grid, EW_THREADS, 0, st>>>(A[0], A[1], A[2], B[0], B[1], B[2], C[0], C[1], C[2], p->wfull,
+  launch_dependent(prodvec_energy_kernel, grid, EW_THREADS, 0, st, A[0], A[1], A[2], B[0], B[1], B[2], C[0], C[1], C[2], p->wfull,
                                                      p->d_z, p->nlat, p->nphi, p->N, scale, acc);
   SPH_LAUNCH_OK();
   return SPH_OK;

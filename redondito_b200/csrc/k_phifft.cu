@@ -55,6 +55,7 @@ struct PhiArgs {
 // the other index with a constant stride, so no runtime divisions remain.
 template <int N, int NP>
 __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd_ct(PhiArgs a) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   constexpr int Q = 2 * NP;             // rings per CTA
   constexpr int JSTEP = PTHREADS / Q;   // phi stride of one thread
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd_ct(PhiArgs a) {
 
 template <int N, int NP>
 __global__ void __launch_bounds__(PTHREADS, 2) phi_inv_ct(PhiArgs a) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   constexpr int Q = 2 * NP;
   constexpr int JSTEP = PTHREADS / Q;
@@ -218,6 +220,7 @@ __device__ __noinline__ void phi_gen_last(const double2* src, double* ring, doub
 constexpr int GENT = 320;  // most threads of the general-length kernels
 
 __global__ void __launch_bounds__(GENT, 2) phi_fwd_gen(PhiArgs a, int lg) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   const int NB = 1 << lg, n = a.nphi, nlat = a.nlat, p0 = blockIdx.x << lg, tid = threadIdx.x;
   const int k = a.kzl ? __ldg(a.kzl + blockIdx.y) : blockIdx.y, f = blockIdx.z;
@@ -257,6 +260,7 @@ __global__ void __launch_bounds__(GENT, 2) phi_fwd_gen(PhiArgs a, int lg) {
 }
 
 __global__ void __launch_bounds__(GENT, 2) phi_inv_gen(PhiArgs a, int lg) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   const int NB = 1 << lg, n = a.nphi, nlat = a.nlat, p0 = blockIdx.x << lg, tid = threadIdx.x;
   const int k = a.kzl ? __ldg(a.kzl + blockIdx.y) : blockIdx.y, f = blockIdx.z;
@@ -339,6 +343,7 @@ bool phi_gen_geometry(const sph_plan* p, int* lg, int* threads, size_t* smem) {
 
 // the in-place engine: lengths whose two buffers do not fit shared memory
 __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd_kernel(PhiArgs a) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   const int NP = a.NP, nphi = a.nphi, nlat = a.nlat, nlat2 = a.nlat2;
   const int p0 = blockIdx.x * NP;
@@ -376,6 +381,7 @@ __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd_kernel(PhiArgs a) {
 }
 
 __global__ void __launch_bounds__(PTHREADS, 2) phi_inv_kernel(PhiArgs a) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   const int NP = a.NP, nphi = a.nphi, nlat = a.nlat, nlat2 = a.nlat2;
   const int p0 = blockIdx.x * NP;
@@ -462,6 +468,7 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 
 template <int N, int NP>
 __global__ void __launch_bounds__(P3d<N, NP>::THREADS, P3d<N, NP>::MINB) phi3_inv64(PhiArgs a, int ntiles) {
+  grid_dependency_wait();
   using G = P3d<N, NP>;
   constexpr int A = G::A, M = G::M, B = G::B, C = G::C, T = G::THREADS;
   extern __shared__ __align__(1024) unsigned char sm3d[];
@@ -579,7 +586,7 @@ int phi3d_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return SPH_ECUDA;
     const int grid = (int)std::min<long long>(ntiles, (long long)occ * std::max(1, nsm));
-    kern<<<grid, G::THREADS, smem, st>>>(a, (int)ntiles);
+    launch_dependent(kern, grid, G::THREADS, smem, st, a, (int)ntiles);
     SPH_LAUNCH_OK();
     return SPH_OK;
   }
@@ -670,6 +677,7 @@ struct GridMaps {
 template <int N, int CL>
 __global__ void __launch_bounds__(P3c<N, CL>::THREADS, P3c<N, CL>::MINB)
     phi3c_fwd64(PhiArgs a, int ntiles, const __grid_constant__ GridMaps maps) {
+  grid_dependency_wait();
   using G = P3c<N, CL>;
   constexpr int A = G::A, M = G::M, B = G::B, C = G::C, T = G::THREADS, NPL = G::NPL, NPC = G::NPC;
   constexpr int ROWS = G::ROWS, BR = G::BR;
@@ -897,11 +905,13 @@ int phi3c_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
         }))
       return SPH_ECUDA;
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = CL;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.blockDim = dim3(G::THREADS);
     cfg.dynamicSmemBytes = G::SMEM;
     cfg.stream = st;
@@ -920,6 +930,7 @@ int phi3c_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
     }
     const long long ncl = std::min<long long>(nclusters, (ntiles + 0));
     cfg.gridDim = dim3((unsigned)(ncl * CL));
+    cfg.numAttrs = 2;  // a dependent launch
     if (cudaLaunchKernelEx(&cfg, kern, a, (int)ntiles, maps) != cudaSuccess) return SPH_ECUDA;
     return SPH_OK;
   }
@@ -957,7 +968,7 @@ bool smem_attr() {
 template <auto KERNEL>
 int run(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
   if (!smem_attr<KERNEL>()) return SPH_ECUDA;
-  KERNEL<<<grid, PTHREADS, smem, st>>>(a);
+  launch_dependent(KERNEL, grid, PTHREADS, smem, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -1041,7 +1052,7 @@ int launch_phi_fwd(const sph_plan* p, const double* const* grids, int nfields, c
   if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run<phi_fwd_kernel>(a, grid, smem, st);
   if (!smem_attr<phi_fwd_gen>()) return SPH_ECUDA;
   grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
-  phi_fwd_gen<<<grid, threads, gsmem, st>>>(a, lg);
+  launch_dependent(phi_fwd_gen, grid, threads, gsmem, st, a, lg);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -1076,7 +1087,7 @@ int launch_phi_inv(const sph_plan* p, double* const* grids, int nfields, cudaStr
   if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run<phi_inv_kernel>(a, grid, smem, st);
   if (!smem_attr<phi_inv_gen>()) return SPH_ECUDA;
   grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
-  phi_inv_gen<<<grid, threads, gsmem, st>>>(a, lg);
+  launch_dependent(phi_inv_gen, grid, threads, gsmem, st, a, lg);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }

@@ -135,6 +135,7 @@ __device__ __forceinline__ void zspectral_store(const ZArgs& a, int r, int lm, s
 
 template <int MODE, int CTN, int IO>
 __global__ void __launch_bounds__(ZTHREADS) zfft_kernel(ZArgs a) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   const int LB = a.LB, nz = a.nz, nlm = a.nlm;
   const int lm0 = blockIdx.x * LB;
@@ -333,6 +334,7 @@ __device__ __forceinline__ void zfft2_body(const ZArgs& a, int blk) {
 template <int MODE, int R1, int R2, int IO>
 __global__ void __launch_bounds__(Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::THREADS,
                                   Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::MINB) zfft2_kernel(ZArgs a) {
+  grid_dependency_wait();
   zfft2_body<MODE, R1, R2, IO>(a, blockIdx.x);
 }
 
@@ -342,6 +344,7 @@ template <int MODE, int R1, int R2, int IO>
 __global__ void __launch_bounds__(Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::THREADS,
                                   Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::MINB)
     zfft2_group_kernel(const ZArgs* __restrict__ jobs, const int* __restrict__ prefix, int njobs) {
+  grid_dependency_wait();
   int lo = 0, hi = njobs - 1;  // last job whose first CTA is <= blockIdx.x
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -366,6 +369,7 @@ __global__ void __launch_bounds__(Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::THR
 // flips there, so another order of the FP64 sums moves their results by 3e-6.
 template <int MODE, int IO, bool DIGITS>
 __global__ void __launch_bounds__(ZTHREADS, DIGITS ? 4 : 2) zfft_gen_kernel(ZArgs a, int lg) {
+  grid_dependency_wait();
   extern __shared__ double2 sm[];
   const int LB = 1 << lg, nz = a.nz, nlm = a.nlm, lm0 = blockIdx.x << lg, tid = threadIdx.x;
   const bool cont = MODE != Z_INV && a.C > 0;
@@ -445,7 +449,7 @@ int launch_gen_as(const ZArgs& a, cudaStream_t st) {
   int lg = 0;
   while ((1 << lg) < a.LB) ++lg;
   const size_t smem = ((size_t)a.nz << lg) * sizeof(double2) * (a.nbuf + zkeep(MODE));
-  zfft_gen_kernel<MODE, IO, DIGITS><<<(a.nlm + a.LB - 1) / a.LB, ZTHREADS, smem, st>>>(a, lg);
+  launch_dependent(zfft_gen_kernel<MODE, IO, DIGITS>, (a.nlm + a.LB - 1) / a.LB, ZTHREADS, smem, st, a, lg);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -475,7 +479,7 @@ int launch_split(const ZArgs& a, int nblocks, cudaStream_t st) {
       }))
     return SPH_ECUDA;
   const size_t smem = (size_t)GZ::LB * R1 * R2 * sizeof(double2) * (zkeep(MODE) ? 2 : 1);
-  zfft2_kernel<MODE, R1, R2, IO><<<nblocks, GZ::THREADS, smem, st>>>(a);
+  launch_dependent(zfft2_kernel<MODE, R1, R2, IO>, nblocks, GZ::THREADS, smem, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -495,7 +499,7 @@ int launch_ct(const ZArgs& a, int nblocks, size_t smem, cudaStream_t st) {
     using GZ = Z2Geo<MODE, CTN, ct::split2_tpc(CTN)>;
     if (a.LB == GZ::LB) return launch_split<MODE, R1, R2, IO>(a, nblocks, st);
   }
-  zfft_kernel<MODE, CTN, IO><<<nblocks, ZTHREADS, smem, st>>>(a);
+  launch_dependent(zfft_kernel<MODE, CTN, IO>, nblocks, ZTHREADS, smem, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }

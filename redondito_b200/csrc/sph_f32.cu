@@ -30,10 +30,12 @@ inline cudaStream_t st_of(void* s) { return (cudaStream_t)s; }
 inline bool f32_ok(const sph_plan* p) { return p && p->precision == SPH_MIXED && slab_whole(p); }
 
 __global__ void widen_kernel(const float* __restrict__ in, double* __restrict__ out, size_t n) {
+  grid_dependency_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = (double)__ldg(in + i);
 }
 __global__ void narrow_kernel(const double* __restrict__ in, float* __restrict__ out, size_t n) {
+  grid_dependency_wait();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = (float)__ldg(in + i);
 }
@@ -43,13 +45,13 @@ int blocks_for(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 1
 // n reals float -> FP64 / FP64 -> float
 int widen(const float* in, double* out, size_t n, cudaStream_t st) {
   if (n == 0) return SPH_OK;
-  widen_kernel<<<blocks_for(n), 256, 0, st>>>(in, out, n);
+  launch_dependent(widen_kernel, blocks_for(n), 256, 0, st, in, out, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
 int narrow(const double* in, float* out, size_t n, cudaStream_t st) {
   if (n == 0) return SPH_OK;
-  narrow_kernel<<<blocks_for(n), 256, 0, st>>>(in, out, n);
+  launch_dependent(narrow_kernel, blocks_for(n), 256, 0, st, in, out, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -66,6 +68,7 @@ int scratch(sph_plan* p, int i, double2** out) {
 // (pseudospec_hd.f90:138-251,291-366; boundary_mod.f90:62-93)
 __global__ void laplang_f32(const float2* __restrict__ a, float2* __restrict__ b, const int* __restrict__ ell,
                             int nlm, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     const int l = ell[q % nlm];
     const double f = -(double)(l * (l + 1));
@@ -75,6 +78,7 @@ __global__ void laplang_f32(const float2* __restrict__ a, float2* __restrict__ b
 }
 __global__ void multr_f32(const float2* __restrict__ a, float2* __restrict__ b, const double* __restrict__ z,
                           int power, int nlm, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
     double zk = z[q / nlm], zp = 1.0;
     const int ap = power < 0 ? -power : power;
@@ -85,12 +89,14 @@ __global__ void multr_f32(const float2* __restrict__ a, float2* __restrict__ b, 
   }
 }
 __global__ void saxpby_f32(float* z, const float* x, double a, const float* y, double b, size_t n) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
     z[q] = (float)(a * (double)x[q] + b * (double)y[q]);
 }
 __global__ void prodvec_f32(const float* __restrict__ ar, const float* __restrict__ at, const float* __restrict__ ap,
                             const float* __restrict__ br, const float* __restrict__ bt, const float* __restrict__ bp,
                             float* cr, float* ct, float* cp, size_t nphys, size_t ntot) {
+  grid_dependency_wait();
   for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < ntot; q += (size_t)gridDim.x * blockDim.x) {
     if (q < nphys) {
       const double xr = ar[q], xt = at[q], xp = ap[q], yr = br[q], yt = bt[q], yp = bp[q];
@@ -103,6 +109,7 @@ __global__ void prodvec_f32(const float* __restrict__ ar, const float* __restric
   }
 }
 __global__ void dirichlet_f32(float2* a, int nlm, int N) {
+  grid_dependency_wait();
   for (int lm = blockIdx.x * blockDim.x + threadIdx.x; lm < nlm; lm += gridDim.x * blockDim.x) {
     a[lm] = make_float2(0.f, 0.f);
     a[(size_t)(N - 1) * nlm + lm] = make_float2(0.f, 0.f);
@@ -295,7 +302,7 @@ extern "C" int sph_fc_filter_f32(sph_plan* p, float* a, char esp, void* s) {
 extern "C" int sph_laplang_f32(sph_plan* p, const float* a, float* b, void* s) {
   if (!f32_ok(p) || !a || !b) return SPH_EINVAL;
   const size_t n = spec_elems(p);
-  laplang_f32<<<blocks_for(n), 256, 0, st_of(s)>>>(reinterpret_cast<const float2*>(a), reinterpret_cast<float2*>(b),
+  launch_dependent(laplang_f32, blocks_for(n), 256, 0, st_of(s), reinterpret_cast<const float2*>(a), reinterpret_cast<float2*>(b),
                                                     p->d_ell, p->nlm, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
@@ -304,7 +311,7 @@ extern "C" int sph_laplang_f32(sph_plan* p, const float* a, float* b, void* s) {
 extern "C" int sph_multr_f32(sph_plan* p, const float* a, float* b, int pw, void* s) {
   if (!f32_ok(p) || !a || !b) return SPH_EINVAL;
   const size_t n = spec_elems(p);
-  multr_f32<<<blocks_for(n), 256, 0, st_of(s)>>>(reinterpret_cast<const float2*>(a), reinterpret_cast<float2*>(b),
+  launch_dependent(multr_f32, blocks_for(n), 256, 0, st_of(s), reinterpret_cast<const float2*>(a), reinterpret_cast<float2*>(b),
                                                   p->d_z, pw, p->nlm, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
@@ -313,7 +320,7 @@ extern "C" int sph_multr_f32(sph_plan* p, const float* a, float* b, int pw, void
 extern "C" int sph_saxpby_c_f32(sph_plan* p, float* z, const float* x, double a, const float* y, double b, void* s) {
   if (!f32_ok(p) || !z || !x || !y) return SPH_EINVAL;
   const size_t n = 2 * spec_elems(p);
-  saxpby_f32<<<blocks_for(n), 256, 0, st_of(s)>>>(z, x, a, y, b, n);
+  launch_dependent(saxpby_f32, blocks_for(n), 256, 0, st_of(s), z, x, a, y, b, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -321,7 +328,7 @@ extern "C" int sph_saxpby_c_f32(sph_plan* p, float* z, const float* x, double a,
 extern "C" int sph_saxpby_r_f32(sph_plan* p, float* z, const float* x, double a, const float* y, double b, void* s) {
   if (!f32_ok(p) || !z || !x || !y) return SPH_EINVAL;
   const size_t n = grid_elems(p);
-  saxpby_f32<<<blocks_for(n), 256, 0, st_of(s)>>>(z, x, a, y, b, n);
+  launch_dependent(saxpby_f32, blocks_for(n), 256, 0, st_of(s), z, x, a, y, b, n);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -338,14 +345,14 @@ extern "C" int sph_prodvec_f32(sph_plan* p, const float* ar, const float* at, co
                                const float* bt, const float* bp, float* cr, float* ct, float* cp, void* s) {
   if (!f32_ok(p) || !ar || !at || !ap || !br || !bt || !bp || !cr || !ct || !cp) return SPH_EINVAL;
   const size_t plane = (size_t)p->nlat * p->nphi, ntot = plane * p->nz, nphys = plane * p->N;
-  prodvec_f32<<<blocks_for(ntot), 256, 0, st_of(s)>>>(ar, at, ap, br, bt, bp, cr, ct, cp, nphys, ntot);
+  launch_dependent(prodvec_f32, blocks_for(ntot), 256, 0, st_of(s), ar, at, ap, br, bt, bp, cr, ct, cp, nphys, ntot);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
 
 extern "C" int sph_dirichlet_f32(sph_plan* p, float* a, void* s) {
   if (!f32_ok(p) || !a) return SPH_EINVAL;
-  dirichlet_f32<<<blocks_for(p->nlm), 256, 0, st_of(s)>>>(reinterpret_cast<float2*>(a), p->nlm, p->N);
+  launch_dependent(dirichlet_f32, blocks_for(p->nlm), 256, 0, st_of(s), reinterpret_cast<float2*>(a), p->nlm, p->N);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }

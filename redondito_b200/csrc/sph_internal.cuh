@@ -407,6 +407,33 @@ int launch_zinv_tiles_g(const sph_plan* p, const void* in, int field, cudaStream
 // the tensor-core synthesis from tiles already in place
 int launch_tc_synthesis_tiles(const sph_plan* p, int vector, cudaStream_t st);
 
+// Dependent launches: a kernel's launch work overlaps the end of the kernel
+// before it on the stream, and every kernel here begins by waiting until that
+// kernel has finished and its writes are visible, so the order of the work is
+// that of plain launches.  (Every CTA waits, also those with nothing to do:
+// the kernel after this one relies on it.)  No kernel triggers its dependent
+// early: waiting CTAs that share an SM with working ones cost more than they
+// saved.  Per pass, plain / this / with early triggers: 5 kernels of a small
+// shell 32.8 / 23.6 / 28.5 us, 7 of a mixed pair 50.5 / 35.9 / 44.1, 12 of a
+// vector pair at lmax 127 285 / 258 / 275, the right-hand sides at lmax 255
+// (mixed) 2949 / 2897 / 3245.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// kernel<<<grid, block, smem, st>>>(args...) as a dependent launch
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 // Runs a set-up step (typically cudaFuncSetAttribute: a kernel's dynamic
 // shared-memory limit) once per device.  Function attributes belong to the
 // context of the device current at the call, so a process that drives

@@ -122,6 +122,7 @@ __global__ void spectrum_kernel(const double2* __restrict__ Z, const double2* __
                                 const double2* __restrict__ Wp, const int* __restrict__ ell,
                                 const int* __restrict__ mbase, const double* __restrict__ z, int lmax, int nlm,
                                 int N, double dz, double* spec) {
+  grid_dependency_wait();
   for (int lm = blockIdx.x * blockDim.x + threadIdx.x; lm < nlm; lm += gridDim.x * blockDim.x) {
     const int l = ell[lm];
     int m = 0;
