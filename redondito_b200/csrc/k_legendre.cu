@@ -358,15 +358,16 @@ __global__ void __launch_bounds__(128, 4) leg_synthesis_kernel(LegArgs a0, LegGr
 }
 
 // ================================================================ vector analysis
-// CTA: 64 consecutive l x 32 planes; K tile 16 nodes.  8 warps = (parity,
+// CTA: 64 consecutive l x 16 planes; K tile 16 nodes.  4 warps = (parity,
 // group of 8 planes), each both outputs of 32 l:
 //   l(l+1) S_re =  dP Vt'_re + mPs Vp_im     l(l+1) S_im =  dP Vt'_im - mPs Vp_re
 //   l(l+1) T_re = -dP Vp'_re + mPs Vt_im     l(l+1) T_im = -dP Vp'_im - mPs Vt_re
 // (' = fold 1 - p, else fold p); -T is accumulated.  Two stages: one K tile
-// is 4096 cycles of tensor work per CTA, more than a load's latency.
-// lmax 511, 256 planes: 8.42 -> 6.66 ms (31.0 TF/s, 84%).
+// is 2048 cycles of tensor work per CTA, more than a load's latency.
+// lmax 511, 256 planes: 8.42 -> 6.55 ms (31.5 TF/s, 85%), with 8 warps and 32
+// planes per CTA 6.65; lmax 255, 10 planes: 181 -> 82 us, 137 with 32.
 namespace va {
-constexpr int L = 64, KZ = 32, K = 16, STAGES = 2;
+constexpr int L = 64, KZ = 16, K = 16, STAGES = 2, THREADS = 8 * KZ;
 constexpr int A_B = 2 * L * ROW, B_B = 8 * KZ * ROW;  // [table][l]; [field][fold][8 nodes][plane]
 constexpr int STAGE = A_B + B_B;
 constexpr int CP = L + 1;
@@ -374,7 +375,7 @@ constexpr int SMEM = STAGES * STAGE;
 static_assert(2 * KZ * CP * 16 <= SMEM, "output staging");
 }  // namespace va
 
-__global__ void __launch_bounds__(256, 2) vec_analysis_kernel(LegArgs a) {
+__global__ void __launch_bounds__(va::THREADS, 4) vec_analysis_kernel(LegArgs a) {
   grid_dependency_wait();
   using namespace va;
   extern __shared__ __align__(128) unsigned char sm[];
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(256, 2) vec_analysis_kernel(LegArgs a) {
   const LegTile tile = a.tiles[bx];
   const int m = tile.m, l0 = tile.r0, kz0 = by * KZ;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int par = warp >> 2, gr = warp & 3;
+  const int par = warp / (KZ / 8), gr = warp % (KZ / 8);
   const size_t base_lm = (size_t)a.mbase[m] - m;
   const int nk = (a.ldn + K - 1) / K;
 
@@ -398,10 +399,11 @@ __global__ void __launch_bounds__(256, 2) vec_analysis_kernel(LegArgs a) {
   auto load = [&](int st, int k0) {
     const bool oka = k0 + 2 * lc < a.ldn;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {  // (table, half of the rows)
-      const bool ok = oka && 32 * (j & 1) <= na;
-      const double* tab = j >> 1 ? a.mPs : a.dP;
-      cp16(da + st * STAGE + j * 32 * ROW, ok ? tab + arow + (size_t)(32 * (j & 1)) * a.ldn + k0 : a.dP, ok);
+    for (int j = 0; j < 2 * (L / KZ); ++j) {  // (table, block of KZ rows)
+      const int r = j % (L / KZ) * KZ;
+      const bool ok = oka && r <= na;
+      const double* tab = j / (L / KZ) ? a.mPs : a.dP;
+      cp16(da + st * STAGE + j * KZ * ROW, ok ? tab + arow + (size_t)r * a.ldn + k0 : a.dP, ok);
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {  // (field, fold, block of 8 nodes)
@@ -473,7 +475,7 @@ __global__ void __launch_bounds__(256, 2) vec_analysis_kernel(LegArgs a) {
     }
   __syncthreads();
   const int nvalid = min(L, a.lmax + 1 - l0);
-  for (int idx = tid; idx < 2 * KZ * L; idx += 256) {
+  for (int idx = tid; idx < 2 * KZ * L; idx += THREADS) {
     const int ll = idx % L, r = idx / L, pl = r % KZ, o = r / KZ;
     bool okz;
     const int kz = plane_of(a, kz0 + pl, okz);
@@ -489,20 +491,21 @@ __global__ void __launch_bounds__(256, 2) vec_analysis_kernel(LegArgs a) {
 }
 
 // ================================================================ vector synthesis
-// CTA: 32 nodes x 32 planes; K tile 16 consecutive l.  8 warps = (fold q,
+// CTA: 32 nodes x 16 planes; K tile 16 consecutive l.  4 warps = (fold q,
 // group of 8 planes), each both outputs of the 32 nodes:
 //   Vt_re =  dP S_re - mPs T_im     Vt_im =  dP S_im + mPs T_re
 //   Vp_re = -dP T_re - mPs S_im     Vp_im = -dP T_im + mPs S_re
 // (rows of parity 1 - q through dP, of parity q through mPs); -Vp is accumulated.
-// lmax 511, 256 planes: 7.41 -> 6.65 ms (31.0 TF/s, 84%).
+// lmax 511, 256 planes: 7.41 -> 6.26 ms (33.0 TF/s, 89%), with 8 warps and 32
+// planes per CTA 6.64; lmax 255, 10 planes: 128 -> 60 us, 108 with 32.
 namespace vs {
-constexpr int I = 32, KZ = 32, K = 16, STAGES = 4;
+constexpr int I = 32, KZ = 16, K = 16, STAGES = 3, THREADS = 8 * KZ;
 constexpr int A_B = 2 * (I / 16) * K * ROW, B_B = 4 * KZ * ROW;  // [table][16 nodes][l]; [S, T][8 l][plane]
 constexpr int STAGE = A_B + B_B;
 constexpr int SMEM = STAGES * STAGE;
 }  // namespace vs
 
-__global__ void __launch_bounds__(256, 2) vec_synthesis_kernel(LegArgs a) {
+__global__ void __launch_bounds__(vs::THREADS, 4) vec_synthesis_kernel(LegArgs a) {
   grid_dependency_wait();
   using namespace vs;
   extern __shared__ __align__(128) unsigned char sm[];
@@ -510,24 +513,24 @@ __global__ void __launch_bounds__(256, 2) vec_synthesis_kernel(LegArgs a) {
   const LegTile tile = a.tiles[bx];
   const int m = tile.m, i0 = tile.r0, kz0 = by * KZ;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int q = warp >> 2, gr = warp & 3;
+  const int q = warp / (KZ / 8), gr = warp % (KZ / 8);
   const size_t base_lm = (size_t)a.mbase[m];
   const int nl = a.lmax + 1 - m, nk = (nl + K - 1) / K;
 
-  const int lc = tid & 7, ar = (tid >> 3) & 15, anb = tid >> 7, bp = tid >> 3;
-  const int ia = i0 + anb * 16 + 2 * lc;
+  const int lc = tid & 7, ar = tid >> 3, bp = tid >> 3;
+  const int ia = i0 + 2 * lc;
   const size_t arow = (base_lm + ar) * a.ldn + ia;
   bool okb;
   const int kzb = plane_of(a, kz0 + bp, okb);
   const size_t brow = (size_t)kzb * a.nlm + base_lm + lc;
   const unsigned s0 = (unsigned)__cvta_generic_to_shared(sm);
-  const unsigned da = s0 + (anb * K + ar) * ROW + ((lc ^ (ar & 7)) << 4), db = s0 + A_B + bp * ROW + ((lc ^ (bp & 7)) << 4);
-  const bool oki = ia < a.ldn;
+  const unsigned da = s0 + ar * ROW + ((lc ^ (ar & 7)) << 4), db = s0 + A_B + bp * ROW + ((lc ^ (bp & 7)) << 4);
   auto load = [&](int st, int q0) {
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const bool ok = oki && q0 + ar < nl;
-      cp16(da + st * STAGE + j * 2 * K * ROW, ok ? (j ? a.mPs : a.dP) + arow + (size_t)q0 * a.ldn : a.dP, ok);
+    for (int j = 0; j < 4; ++j) {  // (table, block of 16 nodes)
+      const bool ok = ia + 16 * (j & 1) < a.ldn && q0 + ar < nl;
+      cp16(da + st * STAGE + j * K * ROW, ok ? (j >> 1 ? a.mPs : a.dP) + arow + (size_t)q0 * a.ldn + 16 * (j & 1) : a.dP,
+           ok);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {  // (S or T, block of 8 degrees); degree 0 has no vector part
@@ -658,7 +661,7 @@ int launch_vec_analysis(const sph_plan* p, double2* s, double2* t, cudaStream_t 
   static DeviceOnce once;
   if (!once.run([] { return set_smem(vec_analysis_kernel, va::SMEM); })) return SPH_ECUDA;
   TimedLaunch tl(p, T_VEC_ANA, st);
-  launch_dependent(vec_analysis_kernel, p->ntilesA64 * a.nkb, 256, va::SMEM, st, a);
+  launch_dependent(vec_analysis_kernel, p->ntilesA64 * a.nkb, va::THREADS, va::SMEM, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
@@ -671,7 +674,7 @@ int launch_vec_synthesis(const sph_plan* p, const double2* s, const double2* t, 
   static DeviceOnce once;
   if (!once.run([] { return set_smem(vec_synthesis_kernel, vs::SMEM); })) return SPH_ECUDA;
   TimedLaunch tl(p, T_VEC_SYN, st);
-  launch_dependent(vec_synthesis_kernel, p->ntilesS32 * a.nkb, 256, vs::SMEM, st, a);
+  launch_dependent(vec_synthesis_kernel, p->ntilesS32 * a.nkb, vs::THREADS, vs::SMEM, st, a);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
