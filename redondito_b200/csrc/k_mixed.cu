@@ -814,7 +814,10 @@ struct P3 {
   // inverse: transform area, twiddles, one staged coefficient tile of (lmax + 1) x 2 x NP float2;
   // two CTAs per SM where that fits for every lmax < N/2 (one loads while the other computes)
   __host__ __device__ static size_t smem_inv(int lmax) { return XBYTES + (size_t)N * sizeof(float2) + stage_inv(lmax) * sizeof(float2); }
-  static constexpr int MINB_INV = XBYTES + (size_t)N * sizeof(float2) + (size_t)N * NP * sizeof(float2) <= 113 * 1024 && THREADS <= 512 ? 2 : 1;
+  static constexpr size_t SMEM_INV_MAX = XBYTES + (size_t)N * sizeof(float2) + (size_t)N * NP * sizeof(float2);
+  // and as many more as fit with 96 registers a thread (nphi 192, 384 tiles: two rounds of 296 CTAs before)
+  static constexpr int MINB_INV = SMEM_INV_MAX > 113 * 1024 || THREADS > 512 ? 1 : std::max(2, std::min(
+      227 * 1024 / (int)(SMEM_INV_MAX + 1024), 65536 / (THREADS * 96)));
   __host__ __device__ static int stage_inv(int lmax) { return (lmax + 1) * 2 * NP; }
 };
 

@@ -44,10 +44,16 @@ struct PhiArgs {
   size_t Gfield;
   int nlat, nlat2, ldn, nphi, nz, lmax, NP;
   const int* kzl;  // planes to transform (nullptr: all nz)
+  int nk;          // their number
   const double* wfold;
   FftDesc fd;
   int* flag;  // set when a bounded wait gives up (cluster three-step forward)
 };
+
+// i-th plane of the launch (the 10 planes a mixed plan transforms in FP64 at
+// nphi 768: inverse 59 -> 37, forward 64 -> 43 us per three fields with the
+// three-step kernels, against phi_inv_ct and phi_fwd_ct)
+__device__ __forceinline__ int plane_at(const PhiArgs& a, int i) { return a.kzl ? __ldg(a.kzl + i) : i; }
 
 // ---------------------------------------------------------------- lengths 2^a 3^b
 // N (phi length) and NP (ring pairs per CTA) fixed at compile time: every
@@ -439,6 +445,27 @@ __global__ void __launch_bounds__(PTHREADS, 2) phi_inv_kernel(PhiArgs a) {
 // 8/NP (mod 8), and staged rows swap their parity halves every 4/NP rows.
 constexpr int up_mod16(int x, int r) { return x + (((r - x) % 16) + 16) % 16; }
 
+// Mirrored rows of the last step (B = 16): the frequencies k = ka + A (kb +
+// B kc) of row (ka, kb) and N - k of row (A - ka, B - 1 - kb) run opposite
+// ways in kc.  Pair j < A/2 B: rows (ka, kb) and (ka2, kb2); in the places of
+// ka = 0 its rows kb and B - kb, then those of ka = A/2.  Pair 0 is the two
+// rows that mirror into themselves, (0, 0) with kc into C - kc and (0, B/2).
+template <int A, int B>
+__device__ __forceinline__ void mirrored_rows(int j, int& ka, int& kb, int& ka2, int& kb2) {
+  const int sl = j / (A / 2);
+  ka = j % (A / 2);
+  kb = sl;
+  kb2 = B - 1 - sl;
+  if (ka == 0 && sl < B / 2) {
+    kb2 = sl ? B - sl : B / 2;
+  } else if (ka == 0) {
+    ka = A / 2;
+    kb = sl - B / 2;
+    kb2 = B - 1 - kb;
+  }
+  ka2 = ka ? A - ka : 0;
+}
+
 template <int N, int NP>
 struct P3d {
   static constexpr int A = 16, M = N / A, B = ct::pow2_part_cap16(M), C = M / B;
@@ -449,7 +476,14 @@ struct P3d {
   static constexpr size_t XBYTES = (size_t)NP * SB * sizeof(double2);
   // transform area, twiddles W_N^e, one staged tile for the largest lmax (N/2 - 1)
   static constexpr size_t SMEM_MAX = XBYTES + (size_t)N * sizeof(double2) + (size_t)N * NP * sizeof(double2);
-  static constexpr int MINB = SMEM_MAX <= 113 * 1024 && THREADS <= 512 ? 2 : 1;
+  // as many CTAs per SM as fit with 128 registers a thread, at least two
+  // where shared memory allows (nphi 192, four fields of 64 planes: 31.9 -> 24.7 us)
+  static constexpr int MINB = SMEM_MAX > 113 * 1024 || THREADS > 512 ? 1 : std::max(2, std::min(
+      227 * 1024 / (int)(SMEM_MAX + 1024), 65536 / (THREADS * 128)));
+  // step (C') on pairs of mirrored rows (nphi 768, six launches of three fields: 1847 -> 1795 us; at
+  // nphi 1536 the pairs leave a third of their second round idle, 4.68 against 4.92 ms)
+  static constexpr bool PAIRED = B == 16 && C == 3;
+  static constexpr int PAIRS = A / 2 * B;
   static size_t smem(int lmax) {
     return XBYTES + (size_t)N * sizeof(double2) + (size_t)(lmax + 1) * 2 * NP * sizeof(double2);
   }
@@ -481,7 +515,7 @@ __global__ void __launch_bounds__(P3d<N, NP>::THREADS, P3d<N, NP>::MINB) phi3_in
   const size_t pstride = (size_t)a.nz * a.ldn;  // parity stride of the folded coefficients
   // the coefficients of a tile into the stage, by cp.async (every thread its share)
   auto issue = [&](int tile) {
-    const int g = tile % ngroups, r = tile / ngroups, k = r % a.nz, f = r / a.nz;
+    const int g = tile % ngroups, r = tile / ngroups, k = plane_at(a, r % a.nk), f = r / a.nk;
     const double2* gs = a.Gc + (size_t)f * a.Gfield + (size_t)k * a.ldn + g * NP;
     const int total = (lmax + 1) * 2 * NP;
     for (int q = t; q < total; q += T) {
@@ -492,7 +526,7 @@ __global__ void __launch_bounds__(P3d<N, NP>::THREADS, P3d<N, NP>::MINB) phi3_in
   };
   if ((int)blockIdx.x < ntiles) issue(blockIdx.x);
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int g = tile % ngroups, r = tile / ngroups, k = r % a.nz, f = r / a.nz, p0 = g * NP;
+    const int g = tile % ngroups, r = tile / ngroups, k = plane_at(a, r % a.nk), f = r / a.nk, p0 = g * NP;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();  // the tile's coefficients have landed; the last tile's step (A') is done with X
     auto zin = [&](int m, int b) {
@@ -509,15 +543,54 @@ __global__ void __launch_bounds__(P3d<N, NP>::THREADS, P3d<N, NP>::MINB) phi3_in
     };
     auto conj = [](double2 z) { return make_double2(z.x, -z.y); };
     // (C')
-    for (int it = t; it < G::ITEMS_C; it += T) {
-      const int b = it % NP, rr = it / NP, ka = rr % A, kb = rr / A;
-      double2 u[C];
-#pragma unroll
-      for (int kc = 0; kc < C; ++kc) u[kc] = zin(ka + A * (kb + B * kc), b);
+    auto put = [&](int b, int ka, int kb, double2 (&u)[C]) {
       ct::RD<double2, C, 1>::run(u);
       double2* row = X + b * G::SB + ka * G::PR + C * kb;
 #pragma unroll
       for (int c = 0; c < C; ++c) row[c] = (c && kb) ? ct::mul(u[c], conj(tw[A * c * kb])) : u[c];
+    };
+    if constexpr (!G::PAIRED) {
+      for (int it = t; it < G::ITEMS_C; it += T) {
+        const int b = it % NP, rr = it / NP, ka = rr % A, kb = rr / A;
+        double2 u[C];
+#pragma unroll
+        for (int kc = 0; kc < C; ++kc) u[kc] = zin(ka + A * (kb + B * kc), b);
+        put(b, ka, kb, u);
+      }
+    } else {  // two mirrored rows from one read of their coefficients
+#pragma unroll 1
+      for (int it = t; it < G::PAIRS * NP; it += T) {
+        const int b = it % NP;
+        int ka, kb, ka2, kb2;
+        mirrored_rows<A, B>(it / NP, ka, kb, ka2, kb2);
+        double2 u[C], v[C];
+        if (it < NP) {
+#pragma unroll
+          for (int kc = 0; kc < C; ++kc) {
+            u[kc] = zin(A * B * kc, b);
+            v[kc] = zin(A * (B / 2 + B * kc), b);
+          }
+        } else {
+#pragma unroll
+          for (int kc = 0; kc < C; ++kc) {
+            const int kk = ka + A * (kb + B * kc);
+            const bool lo = 2 * kk < N;
+            const int m = lo ? kk : N - kk;
+            double2 zl = make_double2(0.0, 0.0), zh = zl;
+            if (m <= lmax) {
+              const int sw = stage_swz64<NP>(m);
+              const double2 se = st[m * 2 * NP + sw * NP + b], so = st[m * 2 * NP + (1 - sw) * NP + b];
+              const double2 Fi = cadd(se, so), Fm = csub(se, so);
+              zl = make_double2(Fi.x - Fm.y, Fi.y + Fm.x);
+              zh = make_double2(Fi.x + Fm.y, -Fi.y + Fm.x);
+            }
+            u[kc] = lo ? zl : zh;
+            v[C - 1 - kc] = lo ? zh : zl;
+          }
+        }
+        put(b, ka, kb, u);
+        put(b, ka2, kb2, v);
+      }
     }
     __syncthreads();
     // step (C') was the last reader of the stage: the next tile's
@@ -575,7 +648,7 @@ int phi3d_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
   } else {
     using G = P3d<N, NP>;
     const size_t smem = G::smem(p->lmax);
-    const long long ntiles = (long long)(p->nlat2 / NP) * p->nz * nfields;
+    const long long ntiles = (long long)(p->nlat2 / NP) * a.nk * nfields;
     if (ntiles == 0) return SPH_OK;
     if (ntiles > (1ll << 30)) return PHI3D_UNSUPPORTED;
     auto kern = phi3_inv64<N, NP>;
@@ -641,7 +714,7 @@ struct P3c {
   // at nphi 384, where a third of the CTA would sit out step (C), 101 against
   // 99 us)
   static constexpr bool PAIRED = B == 16;
-  static constexpr int PAIRS = A / 2 * B;  // pairs of mirrored rows (ka, kb)
+  static constexpr int PAIRS = A / 2 * B;
   static constexpr int PR = M | 1;
   static constexpr int SB = up_mod16(A * PR, 8 / NPL);
   static constexpr size_t XBYTES = (size_t)NPL * SB * sizeof(double2);
@@ -702,7 +775,7 @@ __global__ void __launch_bounds__(P3c<N, CL>::THREADS, P3c<N, CL>::MINB)
   auto stage = [&](int w) { return sm3c + (size_t)w * G::STAGE; };
   // one thread: this CTA's rows of a tile, rings then mirrors
   auto issue = [&](int tile, int w) {
-    const int g = tile % ngroups, r = tile / ngroups, k = r % a.nz, f = r / a.nz;
+    const int g = tile % ngroups, r = tile / ngroups, k = plane_at(a, r % a.nk), f = r / a.nk;
     unsigned char* st = stage(w);
     tma::expect_tx(&full[w], (uint32_t)G::TILE_BYTES);
     const int y0 = k * N + (int)rank * ROWS;
@@ -739,7 +812,7 @@ __global__ void __launch_bounds__(P3c<N, CL>::THREADS, P3c<N, CL>::MINB)
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       issue(tile + ncl, s ^ 1);
     }
-    const int g = tile % ngroups, rr = tile / ngroups, k = rr % a.nz, f = rr / a.nz;
+    const int g = tile % ngroups, rr = tile / ngroups, k = plane_at(a, rr % a.nk), f = rr / a.nk;
     // (A) the samples x[nm + M n1] of local ring pair b (ring: real part, mirror: imaginary part)
     const bool act = t < G::ITEMS_A;
     // ring pair b of the CTA, row nm: with clusters of 2 a staged row is 64
@@ -834,20 +907,11 @@ __global__ void __launch_bounds__(P3c<N, CL>::THREADS, P3c<N, CL>::MINB)
         };
 #pragma unroll 1
         for (int j = (t - 32) / NPL; j < G::PAIRS; j += (T - 32) / NPL) {
-          // rows (ka, kb) and (A - ka, B - 1 - kb); in the places of ka = 0
-          // its rows kb and B - kb, then those of ka = A/2
-          const int sl = j / (A / 2);
-          int ka = j % (A / 2), kb = sl, kb2 = B - 1 - sl;
-          if (ka == 0 && sl < B / 2) {
-            kb2 = sl ? B - sl : B / 2;
-          } else if (ka == 0) {
-            ka = A / 2;
-            kb = sl - B / 2;
-            kb2 = B - 1 - kb;
-          }
+          int ka, kb, ka2, kb2;
+          mirrored_rows<A, B>(j, ka, kb, ka2, kb2);
           double2 u[C], v[C];
           load(ka, kb, u);
-          load(ka ? A - ka : 0, kb2, v);
+          load(ka2, kb2, v);
           if (ka == 0 && kb == 0) {  // two rows that mirror into themselves, the first kc into C - kc
             emit(0, u[0], u[0]);
 #pragma unroll
@@ -885,7 +949,7 @@ int phi3c_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
   } else {
     using G = P3c<N, CL>;
     if (p->nlat2 % G::NPC || !a.flag) return PHI3C_UNSUPPORTED;
-    const long long ntiles = (long long)(p->nlat2 / G::NPC) * p->nz * nfields;
+    const long long ntiles = (long long)(p->nlat2 / G::NPC) * a.nk * nfields;
     if (ntiles == 0) return SPH_OK;
     if (ntiles > (1ll << 30) || (long long)N * p->nz > (1ll << 31) - 1) return PHI3C_UNSUPPORTED;
     GridMaps maps;
@@ -1016,6 +1080,7 @@ PhiArgs make_args(const sph_plan* p) {
   a.wfold = p->wfold;
   a.fd = p->fphi;
   a.kzl = p->sel_kz;
+  a.nk = p->sel_kz ? p->sel_n : p->nz;
   return a;
 }
 
@@ -1026,20 +1091,18 @@ int launch_phi_fwd(const sph_plan* p, const double* const* grids, int nfields, c
   if (p->nphi > PMAXC) return SPH_EINVAL;
   PhiArgs a = make_args(p);
   for (int f = 0; f < nfields; ++f) a.gin[f] = grids[f];
-  dim3 grid(p->nlat2 / a.NP, p->sel_kz ? p->sel_n : p->nz, nfields);
+  dim3 grid(p->nlat2 / a.NP, a.nk, nfields);
   size_t smem = (size_t)a.NP * seq_stride(p->nphi) * sizeof(double2);
   TimedLaunch tl(p, T_PHI_FWD, st);
-  if (!p->sel_kz) {  // the cluster three-step kernel walks every plane
-    a.flag = p->dflag;
-    int rc = PHI3C_UNSUPPORTED;
-    switch (p->nphi) {
+  a.flag = p->dflag;
+  int rc = PHI3C_UNSUPPORTED;
+  switch (p->nphi) {
 #define CASE(n) \
   case n: rc = phi3c_dispatch_n<n>(p, a, nfields, st); break;
-      PHI_SIZES(CASE)
+    PHI_SIZES(CASE)
 #undef CASE
-    }
-    if (rc != PHI3C_UNSUPPORTED) return rc;
   }
+  if (rc != PHI3C_UNSUPPORTED) return rc;
   switch (p->nphi) {
 #define CASE(n) \
   case n: return launch_fwd_n<n>(a, grid, smem, st);
@@ -1062,19 +1125,17 @@ int launch_phi_inv(const sph_plan* p, double* const* grids, int nfields, cudaStr
   if (p->nphi > PMAXC) return SPH_EINVAL;
   PhiArgs a = make_args(p);
   for (int f = 0; f < nfields; ++f) a.gout[f] = grids[f];
-  dim3 grid(p->nlat2 / a.NP, p->sel_kz ? p->sel_n : p->nz, nfields);
+  dim3 grid(p->nlat2 / a.NP, a.nk, nfields);
   size_t smem = (size_t)a.NP * seq_stride(p->nphi) * sizeof(double2);
   TimedLaunch tl(p, T_PHI_INV, st);
-  if (!p->sel_kz) {  // the three-step kernel walks every plane
-    int rc = PHI3D_UNSUPPORTED;
-    switch (p->nphi) {
+  int rc = PHI3D_UNSUPPORTED;
+  switch (p->nphi) {
 #define CASE(n) \
   case n: rc = phi3d_dispatch_n<n>(p, a, nfields, st); break;
-      PHI_SIZES(CASE)
+    PHI_SIZES(CASE)
 #undef CASE
-    }
-    if (rc != PHI3D_UNSUPPORTED) return rc;
   }
+  if (rc != PHI3D_UNSUPPORTED) return rc;
   switch (p->nphi) {
 #define CASE(n) \
   case n: return launch_inv_n<n>(a, grid, smem, st);
