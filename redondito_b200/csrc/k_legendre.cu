@@ -83,7 +83,7 @@ struct LegArgs {
   const LegTile* tiles;
   const int* mbase;
   const int* kzl;  // planes to transform (nullptr: all nz)
-  int lmax, ldn, nz, nlm, nkz;
+  int lmax, nlat2, ldn, nz, nlm, nkz;  // nodes past nlat2 are padding: G holds anything there
   int nkb;         // plane blocks of the launch
 };
 
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(128, 4) leg_analysis_kernel(LegArgs a0, LegGro
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {  // (parity, block of 8 nodes)
-      const bool ok = okb && k0 + (j & 1) * 8 + lc < a.ldn;
+      const bool ok = okb && k0 + (j & 1) * 8 + lc < a.nlat2;
       cp16(db + st * STAGE + j * KZ * ROW, ok ? pb + (j >> 1) * parb + k0 + (j & 1) * 8 : a.G, ok);
     }
   };
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(va::THREADS, 4) vec_analysis_kernel(LegArgs a)
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {  // (field, fold, block of 8 nodes)
-      const bool ok = okb && k0 + (j & 1) * 8 + lc < a.ldn;
+      const bool ok = okb && k0 + (j & 1) * 8 + lc < a.nlat2;
       cp16(db + st * STAGE + j * KZ * ROW,
            ok ? pb + (j >> 2) * a.Gfield + ((j >> 1) & 1) * parb + k0 + (j & 1) * 8 : a.G, ok);
     }
@@ -610,6 +610,7 @@ LegArgs base_args(const sph_plan* p, int kz) {
   a.Gfield = p->Gfield;
   a.mbase = p->d_mbase;
   a.lmax = p->lmax;
+  a.nlat2 = p->nlat2;
   a.ldn = p->ldn;
   a.nz = p->nz;
   a.nlm = p->nlm;

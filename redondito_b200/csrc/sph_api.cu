@@ -411,7 +411,7 @@ extern "C" int sph_plan_create(sph_plan** out, int lmax, int nlat, int nphi, int
   p->Gfield = (size_t)(lmax + 1) * 2 * nz * ldn;
   if (rc == SPH_OK && cudaMalloc((void**)&p->G, SPH_MAX_FIELDS * p->Gfield * sizeof(double2)) != cudaSuccess)
     rc = SPH_ENOMEM;
-  // node columns past nlat/2 are never written and must read as zero
+  // zero to begin with (the node columns past nlat/2 are padding that no kernel reads)
   if (rc == SPH_OK && cudaMemset(p->G, 0, SPH_MAX_FIELDS * p->Gfield * sizeof(double2)) != cudaSuccess)
     rc = SPH_ECUDA;
   if (rc == SPH_OK && cudaMalloc((void**)&p->energy, sizeof(double)) != cudaSuccess) rc = SPH_ENOMEM;
