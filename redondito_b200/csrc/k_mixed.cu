@@ -815,9 +815,15 @@ struct P3 {
   // two CTAs per SM where that fits for every lmax < N/2 (one loads while the other computes)
   __host__ __device__ static size_t smem_inv(int lmax) { return XBYTES + (size_t)N * sizeof(float2) + stage_inv(lmax) * sizeof(float2); }
   static constexpr size_t SMEM_INV_MAX = XBYTES + (size_t)N * sizeof(float2) + (size_t)N * NP * sizeof(float2);
-  // and as many more as fit with 96 registers a thread (nphi 192, 384 tiles: two rounds of 296 CTAs before)
-  static constexpr int MINB_INV = SMEM_INV_MAX > 113 * 1024 || THREADS > 512 ? 1 : std::max(2, std::min(
-      227 * 1024 / (int)(SMEM_INV_MAX + 1024), 65536 / (THREADS * 96)));
+  // and as many more as fit with 96 registers a thread (nphi 192, 384 tiles: two rounds of 296 CTAs before;
+  // whole synthesis, 64 planes: nphi 192 51 -> 36 us, 384 101 -> 92), except for long rows of runs of half a
+  // sector (2 ring pairs of FP64 grids, 4 of float ones; see phi_inv_smem): nphi 768, nlat 388, 16 planes
+  // 203 us with seven CTAs, 197 with two and 232 registers; nphi 1536, nlat 772 1092 against 939
+  __host__ __device__ static constexpr int minb_inv(int elem) {
+    return SMEM_INV_MAX > 113 * 1024 || THREADS > 512                             ? 1
+           : (NP * elem == 16 && N >= 768) || (NP * elem < 32 && N >= 1536)       ? 2
+           : std::max(2, std::min(227 * 1024 / (int)(SMEM_INV_MAX + 1024), 65536 / (THREADS * 96)));
+  }
   __host__ __device__ static int stage_inv(int lmax) { return (lmax + 1) * 2 * NP; }
 };
 
@@ -992,7 +998,8 @@ __global__ void __launch_bounds__(P3<N, NP>::THREADS, P3<N, NP>::MINB)
 }
 
 template <int N, int NP, typename GT>
-__global__ void __launch_bounds__(P3<N, NP>::THREADS, P3<N, NP>::MINB_INV) phi3_inv32(Phi32Args a, int ntiles) {
+__global__ void __launch_bounds__(P3<N, NP>::THREADS, P3<N, NP>::minb_inv(sizeof(GT)))
+    phi3_inv32(Phi32Args a, int ntiles) {
   grid_dependency_wait();
   using G = P3<N, NP>;
   constexpr int A = G::A, M = G::M, B = G::B, C = G::C, T = G::THREADS;
@@ -1961,7 +1968,7 @@ int phi3_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
     return PHI3_UNSUPPORTED;
   } else {
     using G = P3<N, NP>;
-    const size_t smem = FWD ? G::SMEM_F : G::smem_inv(p->lmax);
+    size_t smem = FWD ? G::SMEM_F : G::smem_inv(p->lmax);
     if (smem > PHI3_SMEM_MAX) return PHI3_UNSUPPORTED;
     const long long ntiles = (long long)(p->nlat2 / NP) * p->nz * nfields;
     if (ntiles == 0) return SPH_OK;
@@ -1986,6 +1993,7 @@ int phi3_run(const sph_plan* p, const Phi32Args& a, int nfields, cudaStream_t st
       launch_dependent(kern, grid, G::THREADS, smem, st, a, (int)ntiles, maps);
     } else {
       auto kern = phi3_inv32<N, NP, GT>;
+      smem = phi_inv_smem(smem, N, NP * (int)sizeof(GT), (double)grid_elems(p) * nfields * sizeof(GT), L2_BYTES);
       const int occ = residency.get(kern, G::THREADS, smem, PHI3_SMEM_MAX);
       if (!occ) return SPH_ECUDA;
       const int grid = (int)std::min<long long>(ntiles, (long long)occ * std::max(1, p->nsm));

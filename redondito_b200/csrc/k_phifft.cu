@@ -647,13 +647,14 @@ int phi3d_run(const sph_plan* p, const PhiArgs& a, int nfields, cudaStream_t st)
     return PHI3D_UNSUPPORTED;
   } else {
     using G = P3d<N, NP>;
-    const size_t smem = G::smem(p->lmax);
+    const size_t smem = phi_inv_smem(G::smem(p->lmax), N, NP * (int)sizeof(double),
+                                     (double)N * p->nlat * a.nk * nfields * sizeof(double), 2 * L2_BYTES);
     const long long ntiles = (long long)(p->nlat2 / NP) * a.nk * nfields;
     if (ntiles == 0) return SPH_OK;
     if (ntiles > (1ll << 30)) return PHI3D_UNSUPPORTED;
     auto kern = phi3_inv64<N, NP>;
     static Residency residency;
-    const int occ = residency.get(kern, G::THREADS, smem, G::SMEM_MAX);
+    const int occ = residency.get(kern, G::THREADS, smem, std::max<size_t>(G::SMEM_MAX, 80 * 1024));
     int dev = 0, nsm = 0;
     if (!occ || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)

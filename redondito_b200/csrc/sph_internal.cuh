@@ -478,6 +478,25 @@ struct Residency {
   }
 };
 
+// Dynamic shared memory of a launch of the persistent inverse phi kernels,
+// from the `smem` bytes it uses, for tiles that write runs of `run` bytes to
+// each of nphi grid rows.  A run below a 32-byte sector leaves the sector half
+// written in L2 until the neighbouring tile writes the rest; with many such
+// tiles in flight on grids past L2 (`bytes` over `limit`) L2 gives them up
+// before.  Those launches take enough shared memory that four CTAs (nphi 384)
+// or two (768 and above) share an SM.  Whole synthesis of three fields with 2
+// ring pairs per tile, all that fit / so limited: FP64 at nphi 768, nlat 388,
+// 64 planes 767 / 596 us, 128 planes 1796 / 1198 (32 planes, 229 MB, 325 /
+// 321: below its limit of 2 L2); fp32 at nphi 384, nlat 392, 128 planes 279 /
+// 224 (64 planes, 116 MB, 129 / 127); nphi 192 at 236 MB 252 / 265: not
+// limited.
+constexpr double L2_BYTES = 126e6;
+static inline size_t phi_inv_smem(size_t smem, int nphi, int run, double bytes, double limit) {
+  if (run >= 32 || nphi < 384 || bytes <= limit) return smem;
+  const size_t share = (size_t)228 * 1024 / (nphi < 768 ? 5 : 3) + 1;  // one CTA more does not fit
+  return smem < share ? share : smem;
+}
+
 #define SPH_CUDA_OK(call)                     \
   do {                                        \
     cudaError_t e_ = (call);                  \
