@@ -237,7 +237,11 @@ __global__ void __launch_bounds__(ZTHREADS) zfft_kernel(ZArgs a) {
 // in the derivative), so many small CTAs overlap best.  Derivative and D_l of
 // 32896 columns: nz 96 55 and 64 -> 36 and 48 us, nz 128 53 and 66 -> 43 and
 // 64 us, against the spectrum put back in natural order between two full
-// splits, 128-148 registers and 16 columns.
+// splits, 128-148 registers and 16 columns.  The modes that keep the input
+// column take the registers of the CTAs their shared memory lets share an SM
+// (four at nz 192, three at 256), else they spill: D_l of 73920 columns nz 192
+// 232 -> 196 us (217 before the exchange from registers), nz 256 292 -> 194
+// (261).
 __host__ __device__ constexpr int z2_lb(int nz) {
   int lb = 32;
   while (lb > 8 && lb * ct::split2_tpc(nz) > 128) lb >>= 1;
@@ -248,7 +252,8 @@ struct Z2Geo {
   static constexpr int LB = z2_lb(NZ), THREADS = LB * TPC;
   static constexpr bool PLAIN = MODE == Z_FWD || MODE == Z_INV;
   static constexpr int RPT = 84;
-  static constexpr int MINB = 65536 / (THREADS * RPT) > 1 ? 65536 / (THREADS * RPT) : 1;
+  static constexpr int SMEM = LB * NZ * (int)sizeof(double2) * (zkeep(MODE) ? 2 : 1);
+  static constexpr int MINB = std::max(1, std::min(65536 / (THREADS * RPT), 227 * 1024 / (SMEM + 1024)));
 };
 
 // column block blk of the spectra a describes
