@@ -50,8 +50,8 @@ struct ZArgs {
   // the passes of the nonlinear step (Z_POT, Z_RHS, Z_DLADD)
   ZNlArgs nl;
   const double *z, *zinv;  // r, 1/r
-  bool digits;  // general lengths: the passes of fft_engine.cuh
-  int nbuf;     // their buffers: one where every radix is done in place
+  bool digits;  // general lengths: a mixed plan's passes of fft_engine.cuh
+  int nbuf;     // buffers of a general length: one where every radix is done in place
 };
 
 // modes that keep the whole input column (every row) beside the transform's
@@ -368,10 +368,12 @@ __global__ void __launch_bounds__(Z2Geo<MODE, R1 * R2, (R1 > R2 ? R1 : R2)>::THR
 // 14706 columns, plain: 19-27 against 52-59 us.
 //
 // DIGITS: the decimation-in-frequency and -in-time passes of fft_engine.cuh
-// instead, the spectrum in digit-reversed order between them.  Mixed plans
-// take these on FP64 arrays: the fp32 steps after a z transform round, and a
-// forward continuation (weights up to 3.7e3) amplifies what a last-bit change
-// flips there, so another order of the FP64 sums moves their results by 3e-6.
+// instead, the spectrum in digit-reversed order between them.  Wide slabs of
+// some lengths take these (launch_gen), and mixed plans on FP64 arrays: the
+// fp32 steps after a z transform round, and a forward continuation (weights up
+// to 3.7e3) amplifies what a last-bit change flips there, so another order of
+// the FP64 sums moves their results by 3e-6, and a run on a mixed plan would
+// not repeat on another release of the library.
 template <int MODE, int IO, bool DIGITS>
 __global__ void __launch_bounds__(ZTHREADS, DIGITS ? 4 : 2) zfft_gen_kernel(ZArgs a, int lg) {
   grid_dependency_wait();
@@ -441,6 +443,13 @@ int zgen_lb(int nz, int nlm) {
   return lb;
 }
 
+// Shared memory of a zfft_gen_kernel CTA at most, so that two share an SM:
+// wider slabs (tuned widths) are cut to what fits.  D_l of a mixed plan, 8256
+// columns, nz 400 at 8 columns: 407 us uncut, 239 cut to 4; nz 120 at 32
+// columns, derivative, 75 and 53 (345 and 60 with the in-place passes of one
+// thread per butterfly).
+constexpr size_t ZGEN_SMEM = 112 * 1024;
+
 template <int MODE, int IO, bool DIGITS>
 int launch_gen_as(const ZArgs& a, cudaStream_t st) {
   static DeviceOnce once;
@@ -453,22 +462,27 @@ int launch_gen_as(const ZArgs& a, cudaStream_t st) {
     return SPH_ECUDA;
   int lg = 0;
   while ((1 << lg) < a.LB) ++lg;
-  const size_t smem = ((size_t)a.nz << lg) * sizeof(double2) * (a.nbuf + zkeep(MODE));
-  launch_dependent(zfft_gen_kernel<MODE, IO, DIGITS>, (a.nlm + a.LB - 1) / a.LB, ZTHREADS, smem, st, a, lg);
+  const size_t col = (size_t)a.nz * sizeof(double2) * (a.nbuf + zkeep(MODE));
+  while (lg > 0 && (col << lg) > ZGEN_SMEM) --lg;
+  launch_dependent(zfft_gen_kernel<MODE, IO, DIGITS>, (a.nlm + (1 << lg) - 1) >> lg, ZTHREADS, col << lg, st, a, lg);
   SPH_LAUNCH_OK();
   return SPH_OK;
 }
 
+// The in-place passes (DIGITS) also where two buffers of a tuned slab would
+// have to be cut, every radix is 2, 3, 4 or 8 and there are no more passes:
+// one buffer keeps the columns (FP64 derivative, nz 1024 at 4 columns: 8256
+// columns 247 us uncut, 206 in place; 18528 columns 560 uncut, 505 cut).
 template <int MODE, int IO>
 int launch_gen(ZArgs a, cudaStream_t st) {
-  a.nbuf = 2;
-  if constexpr (IO == ZIO_DD)
-    if (a.digits) {
-      a.nbuf = 1;
-      for (int i = 0; i < a.fd.npass; ++i)
-        if (!fft_inplace_radix(a.fd.pass[i].R)) a.nbuf = 2;
-      return launch_gen_as<MODE, IO, true>(a, st);
-    }
+  bool digits = IO == ZIO_DD && a.digits, inplace = true;
+  for (int i = 0; i < a.fd.npass; ++i) inplace = inplace && fft_inplace_radix(a.fd.pass[i].R);
+  if constexpr (!zkeep(MODE))
+    digits = digits || (inplace && a.fd.npass <= a.fd.ng && a.LB > 1 &&
+                        (size_t)a.LB * a.nz * sizeof(double2) * 2 > ZGEN_SMEM);
+  a.nbuf = digits && inplace ? 1 : 2;
+  if constexpr (IO == ZIO_DD || !zkeep(MODE))
+    if (digits) return launch_gen_as<MODE, IO, true>(a, st);
   return launch_gen_as<MODE, IO, false>(a, st);
 }
 

@@ -1,9 +1,19 @@
 """Routes that a rule on sizes chooses: each against the oracle or, where the
 arithmetic is the same, bit for bit against the route beside it."""
+import numpy as np
 import pytest
+
+from oracle import oracle as O
+from tests._helpers import check, random_spec, rel_l2
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
+
+TOL = 1e-12  # the FP64 bound of the transform tests
+
+
+def dev(x):
+    return torch.from_numpy(np.ascontiguousarray(x)).cuda()
 
 
 # The inverse phi transforms with 2 ring pairs per tile on grids past the L2
@@ -31,3 +41,39 @@ def test_inverse_phi_past_l2(form, nlat, nphi, nz):
             assert torch.equal(x[k:k + few], y), f"planes {k}.."
     many.close()
     part.close()
+
+
+# Tuned widths of the general radial lengths past the shared memory of two
+# CTAs per SM: cut to it (58 at 64 columns, 400 at 8, 120 at 32), or, for 1024
+# and 2048, the in-place passes at the full width.
+@pytest.mark.parametrize("nz,cols", [(58, 64), (120, 32), (400, 8), (1024, 4), (2048, 2)])
+@pytest.mark.parametrize("form", ["fp64", "mixed", "f32"])
+def test_wide_slabs(nz, cols, form):
+    from redondito_b200 import sphp as S
+    lmax, nlat, nphi = 7, 24, 48
+    P = O.Plan(lmax, nz, nlat=nlat, nphi=nphi)
+    G, H, M = (S.Plan(lmax, nz, nlat=nlat, nphi=nphi, precision=p)
+               for p in ((S.SPH_FP64, S.SPH_FP64, S.SPH_MIXED) if form == "fp64" else (S.SPH_MIXED,) * 3))
+    S.set_tiles(G, z_cols=cols)
+    a = random_spec(P, np.random.default_rng(nz))
+    f32 = form == "f32"
+    x, b, c = (dev(a.astype(np.complex64 if f32 else np.complex128)) for _ in range(3))
+    tol = 1e-6 if f32 else TOL  # float arrays round to 6e-8
+    call = lambda name: getattr(S, name + ("_f32" if f32 else ""))
+    ref = P.z_forward(x.cpu().numpy().astype(np.complex128))
+    call("fftp1d_real_to_complex_z")(G, x)
+    check(rel_l2(x.cpu().numpy(), ref), tol, f"nz {nz} forward")
+    ref = P.z_inverse(x.cpu().numpy().astype(np.complex128))
+    call("fftp1d_complex_to_real_z")(G, x)
+    check(rel_l2(x.cpu().numpy(), ref), tol, f"nz {nz} inverse")
+    # the operators against the default width, whose engine is the same but
+    # for the in-place derivatives: those are a mixed plan's, of FP64 arrays
+    inplace = nz >= 1024 and form != "mixed"
+    for name, args, plan in (("derivr", (2, "r"), M if inplace else H), ("dlr", (), H)):
+        if inplace and f32 and name == "derivr":
+            continue
+        call(name)(G, b, x, *args)
+        call(name)(plan, b, c, *args)
+        assert torch.equal(x, c), name
+    for plan in (G, H, M):
+        plan.close()
