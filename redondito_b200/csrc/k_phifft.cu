@@ -13,8 +13,8 @@
 // with W_i = w_i 2 pi / nphi; the inverse kernel reads the same layout
 // (synthesised even/odd sums) and writes both rings of the grid.
 // Lengths 3 2^a use compile-time FFTs (fft3.cuh, fft_ct.cuh); others the
-// out-of-place passes of fft_gen.cuh, or, past the length whose two buffers
-// fit shared memory, the in-place engine of fft_engine.cuh.
+// out-of-place passes of fft_gen.cuh or, where phi_gen_geometry says so, the
+// in-place engine of fft_engine.cuh.
 #include <algorithm>
 
 #include "fft3.cuh"
@@ -314,9 +314,10 @@ __global__ void __launch_bounds__(GENT, 2) phi_inv_gen(PhiArgs a, int lg) {
 // Ring pairs and threads per CTA of the general-length kernels: the tuned
 // ring pairs, else the most of 8, 4, 2 and 1 whose two buffers let two CTAs
 // share an SM (longer runs of a grid row against more loads in flight); then
-// the threads that leave the fewest lanes idle over the passes.  False: even
-// one pair's buffers exceed shared memory.
-bool phi_gen_geometry(const sph_plan* p, int* lg, int* threads, size_t* smem) {
+// the threads that leave the fewest lanes idle over the passes.  False: the
+// in-place engine takes the length (one pair's buffers exceed shared memory,
+// or its tile is the better one).
+bool phi_gen_geometry(const sph_plan* p, bool fwd, int* lg, int* threads, size_t* smem) {
   const size_t pair = 2 * (size_t)p->nphi * sizeof(double2);
   int l = 0;
   if (p->tile_np) {
@@ -327,6 +328,19 @@ bool phi_gen_geometry(const sph_plan* p, int* lg, int* threads, size_t* smem) {
     while (l > 0 && (pair << l) > 110 * 1024) --l;
   }
   if ((pair << l) > 200 * 1024) return false;
+  // Where the two buffers leave one ring pair to a CTA and the in-place passes
+  // are as few and all in registers, the in-place engine's tile is the better
+  // one: it holds twice the ring pairs or more, so longer runs of a grid row.
+  // The forward transform, which waits for its reads, gains with a pass more
+  // too where two CTAs do not share an SM.  Three fields of 16 planes, nlat
+  // 256, out of place / in place, inverse and forward: nphi 2048 319 / 290 and
+  // 400 / 314 us, 4096 709 / 580 and 992 / 713; forward 4608 (a pass more)
+  // 1104 / 1006, but 5184 (two more) 1236 / 1264.
+  if (l == 0 && (p->tile_np ? pair : 2 * pair) > 110 * 1024) {
+    bool inplace = p->fphi.npass <= p->fphi.ng + (fwd && pair > 110 * 1024);
+    for (int i = 0; i < p->fphi.npass; ++i) inplace = inplace && fft_inplace_radix(p->fphi.pass[i].R);
+    if (inplace) return false;
+  }
   long long least = 0;
   *threads = 0;
   for (int t = 128; t <= GENT; t += 32) {
@@ -347,7 +361,7 @@ bool phi_gen_geometry(const sph_plan* p, int* lg, int* threads, size_t* smem) {
   return true;
 }
 
-// the in-place engine: lengths whose two buffers do not fit shared memory
+// the in-place engine: the lengths phi_gen_geometry leaves to it
 __global__ void __launch_bounds__(PTHREADS, 2) phi_fwd_kernel(PhiArgs a) {
   grid_dependency_wait();
   extern __shared__ double2 sm[];
@@ -1113,7 +1127,7 @@ int launch_phi_fwd(const sph_plan* p, const double* const* grids, int nfields, c
   }
   int lg = 0, threads = 0;
   size_t gsmem = 0;
-  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run<phi_fwd_kernel>(a, grid, smem, st);
+  if (!phi_gen_geometry(p, true, &lg, &threads, &gsmem)) return run<phi_fwd_kernel>(a, grid, smem, st);
   if (!smem_attr<phi_fwd_gen>()) return SPH_ECUDA;
   grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
   launch_dependent(phi_fwd_gen, grid, threads, gsmem, st, a, lg);
@@ -1146,7 +1160,7 @@ int launch_phi_inv(const sph_plan* p, double* const* grids, int nfields, cudaStr
   }
   int lg = 0, threads = 0;
   size_t gsmem = 0;
-  if (!phi_gen_geometry(p, &lg, &threads, &gsmem)) return run<phi_inv_kernel>(a, grid, smem, st);
+  if (!phi_gen_geometry(p, false, &lg, &threads, &gsmem)) return run<phi_inv_kernel>(a, grid, smem, st);
   if (!smem_attr<phi_inv_gen>()) return SPH_ECUDA;
   grid.x = (p->nlat2 + (1 << lg) - 1) >> lg;
   launch_dependent(phi_inv_gen, grid, threads, gsmem, st, a, lg);

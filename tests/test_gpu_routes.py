@@ -77,3 +77,28 @@ def test_wide_slabs(nz, cols, form):
         assert torch.equal(x, c), name
     for plan in (G, H, M):
         plan.close()
+
+
+# Azimuthal lengths past those that fit two ring pairs: 2048 and 4096 (the
+# in-place engine where two buffers leave one ring pair), 4608 and 6400 (the
+# longest) out of place, 6500 and 8192 whose two buffers do not fit; pairs 1 at
+# 2048 goes out of place; nlat / 2 = 5 and 6 (1 and 2 ring pairs in place)
+@pytest.mark.parametrize("nphi", [2048, 4096, 4608, 6400, 6500, 8192])
+@pytest.mark.parametrize("nlat,pairs", [(10, 0), (12, 0), (12, 1)])
+def test_long_phi_lengths(nphi, nlat, pairs):
+    from redondito_b200 import sphp as S
+    P = O.Plan(5, 2, nlat=nlat, nphi=nphi)
+    G = S.Plan(5, 2, nlat=nlat, nphi=nphi)
+    S.set_tiles(G, ring_pairs=pairs)
+    rng = np.random.default_rng(nphi)
+    q, s, t = (random_spec(P, rng, radial=False) for _ in range(3))
+    ref = P.qst_synthesis(q, s, t)
+    g = [G.new_grid() for _ in range(3)]
+    S.fftp2d_qst_to_vec(G, dev(q), dev(s), dev(t), *g)
+    for x, r in zip(g, ref):
+        check(rel_l2(x.cpu().numpy(), r), TOL, f"nphi {nphi} synthesis")
+    c = [G.new_spec() for _ in range(3)]
+    S.fftp2d_vec_to_qst(G, *(dev(r) for r in ref), *c)
+    for x, r in zip(c, P.qst_analysis(*ref)):
+        check(rel_l2(x.cpu().numpy(), r), TOL, f"nphi {nphi} analysis")
+    G.close()
