@@ -1054,26 +1054,22 @@ int run(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
 
 template <int N>
 int launch_fwd_n(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
-  if constexpr (N > 0) {
-    switch (a.NP) {
-      case 8: if constexpr (8 * N <= PMAXC) return run<phi_fwd_ct<N, 8>>(a, grid, smem, st); break;
-      case 4: if constexpr (4 * N <= PMAXC) return run<phi_fwd_ct<N, 4>>(a, grid, smem, st); break;
-      case 2: if constexpr (2 * N <= PMAXC) return run<phi_fwd_ct<N, 2>>(a, grid, smem, st); break;
-      case 1: return run<phi_fwd_ct<N, 1>>(a, grid, smem, st);
-    }
+  switch (a.NP) {
+    case 8: if constexpr (8 * N <= PMAXC) return run<phi_fwd_ct<N, 8>>(a, grid, smem, st); break;
+    case 4: if constexpr (4 * N <= PMAXC) return run<phi_fwd_ct<N, 4>>(a, grid, smem, st); break;
+    case 2: if constexpr (2 * N <= PMAXC) return run<phi_fwd_ct<N, 2>>(a, grid, smem, st); break;
+    case 1: return run<phi_fwd_ct<N, 1>>(a, grid, smem, st);
   }
   return SPH_EINVAL;
 }
 
 template <int N>
 int launch_inv_n(const PhiArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
-  if constexpr (N > 0) {
-    switch (a.NP) {
-      case 8: if constexpr (8 * N <= PMAXC) return run<phi_inv_ct<N, 8>>(a, grid, smem, st); break;
-      case 4: if constexpr (4 * N <= PMAXC) return run<phi_inv_ct<N, 4>>(a, grid, smem, st); break;
-      case 2: if constexpr (2 * N <= PMAXC) return run<phi_inv_ct<N, 2>>(a, grid, smem, st); break;
-      case 1: return run<phi_inv_ct<N, 1>>(a, grid, smem, st);
-    }
+  switch (a.NP) {
+    case 8: if constexpr (8 * N <= PMAXC) return run<phi_inv_ct<N, 8>>(a, grid, smem, st); break;
+    case 4: if constexpr (4 * N <= PMAXC) return run<phi_inv_ct<N, 4>>(a, grid, smem, st); break;
+    case 2: if constexpr (2 * N <= PMAXC) return run<phi_inv_ct<N, 2>>(a, grid, smem, st); break;
+    case 1: return run<phi_inv_ct<N, 1>>(a, grid, smem, st);
   }
   return SPH_EINVAL;
 }

@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(ZTHREADS, DIGITS ? 4 : 2) zfft_gen_kernel(ZArg
 
 // Columns per CTA of zfft_gen_kernel where the plan sets none: the default
 // slab (32 KB), halved down to 4 columns while the grid has fewer than two
-// CTAs per SM (a 528-column derivative at nz 58 then has 132 CTAs, not 17).
+// CTAs for each of a B200's 148 SMs (a 528-column derivative at nz 58 then has 132 CTAs, not 17).
 int zgen_lb(int nz, int nlm) {
   int lb = 64;
   while (lb > 1 && lb * nz > ZMAXCOL / 2) lb >>= 1;
@@ -505,22 +505,22 @@ int launch_split(const ZArgs& a, int nblocks, cudaStream_t st) {
 
 template <int MODE, int CTN, int IO>
 int launch_ct(const ZArgs& a, int nblocks, size_t smem, cudaStream_t st) {
-  static DeviceOnce once;
-  if (!once.run([] {
-        return cudaFuncSetAttribute(zfft_kernel<MODE, CTN, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    200 * 1024) == cudaSuccess &&
-               cudaFuncSetAttribute(zfft_kernel<MODE, CTN, IO>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    100) == cudaSuccess;
-      }))
-    return SPH_ECUDA;
-  if constexpr (CTN > 0 && ct::split2_r1(CTN) > 0) {
-    constexpr int R1 = ct::split2_r1(CTN), R2 = CTN / R1;
-    using GZ = Z2Geo<MODE, CTN, ct::split2_tpc(CTN)>;
-    if (a.LB == GZ::LB) return launch_split<MODE, R1, R2, IO>(a, nblocks, st);
+  if constexpr (ct::split2_r1(CTN) > 0) {  // a.LB is z2_lb(CTN): widths of these lengths are not tuned
+    constexpr int R1 = ct::split2_r1(CTN);
+    return launch_split<MODE, R1, CTN / R1, IO>(a, nblocks, st);
+  } else {
+    static DeviceOnce once;
+    if (!once.run([] {
+          return cudaFuncSetAttribute(zfft_kernel<MODE, CTN, IO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      200 * 1024) == cudaSuccess &&
+                 cudaFuncSetAttribute(zfft_kernel<MODE, CTN, IO>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      100) == cudaSuccess;
+        }))
+      return SPH_ECUDA;
+    launch_dependent(zfft_kernel<MODE, CTN, IO>, nblocks, ZTHREADS, smem, st, a);
+    SPH_LAUNCH_OK();
+    return SPH_OK;
   }
-  launch_dependent(zfft_kernel<MODE, CTN, IO>, nblocks, ZTHREADS, smem, st, a);
-  SPH_LAUNCH_OK();
-  return SPH_OK;
 }
 
 #define Z_SIZES(X) X(16) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(512)
