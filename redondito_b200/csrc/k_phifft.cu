@@ -494,10 +494,12 @@ struct P3d {
   // where shared memory allows (nphi 192, four fields of 64 planes: 31.9 -> 24.7 us)
   static constexpr int MINB = SMEM_MAX > 113 * 1024 || THREADS > 512 ? 1 : std::max(2, std::min(
       227 * 1024 / (int)(SMEM_MAX + 1024), 65536 / (THREADS * 128)));
-  // step (C') on pairs of mirrored rows (nphi 768, six launches of three fields: 1847 -> 1795 us; at
-  // nphi 1536 the pairs leave a third of their second round idle, 4.68 against 4.92 ms)
-  static constexpr bool PAIRED = B == 16 && C == 3;
+  // step (C') on pairs of mirrored rows where the CTA's rounds over pairs take no more turns than those
+  // over single rows (nphi 768, 8 ring pairs: 3 rounds of 2 rows against 6, six launches of three fields
+  // 1847 -> 1795 us; nphi 1536, 4 ring pairs: 2 of 2 against 3, 4.68 -> 4.92 ms); B < 16 was not measured
   static constexpr int PAIRS = A / 2 * B;
+  static constexpr bool PAIRED =
+      B == 16 && 2 * ((PAIRS * NP + THREADS - 1) / THREADS) <= (ITEMS_C + THREADS - 1) / THREADS;
   static size_t smem(int lmax) {
     return XBYTES + (size_t)N * sizeof(double2) + (size_t)(lmax + 1) * 2 * NP * sizeof(double2);
   }
