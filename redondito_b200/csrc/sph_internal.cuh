@@ -454,26 +454,33 @@ struct DeviceOnce {
 };
 
 // A kernel's CTAs per SM, asked of the driver once per device and amount of
-// shared memory (the kernel's limits are set with it, to `limit` bytes for
-// every amount, so that plans of different sizes launch side by side): the
-// three queries of a launch took longer than the launch.  0: a CUDA error.
+// shared memory, the last four amounts kept (plans of different sizes, and the
+// larger launches of phi_inv_smem, alternate); the kernel's limits are set
+// with it, to `limit` bytes for every amount, so that they launch side by
+// side.  The three queries of a launch took longer than the launch.  0: a CUDA
+// error.
 struct Residency {
-  std::atomic<unsigned long long> seen[64];  // shared memory + 1 in the high bits, CTAs in the low 16
+  static constexpr int KEEP = 4;
+  std::atomic<unsigned long long> seen[64][KEEP];  // shared memory + 1 in the high bits, CTAs in the low 16
+  std::atomic<unsigned> next[64];
   template <typename K>
   int get(K kernel, int threads, size_t smem, size_t limit) {
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     const bool keep = dev >= 0 && dev < 64;
-    if (keep) {
-      const unsigned long long v = seen[dev].load(std::memory_order_acquire);
-      if ((v >> 16) == smem + 1) return (int)(v & 0xffff);
-    }
+    if (keep)
+      for (const auto& s : seen[dev]) {
+        const unsigned long long v = s.load(std::memory_order_acquire);
+        if ((v >> 16) == smem + 1) return (int)(v & 0xffff);
+      }
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit) != cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) != cudaSuccess)
       return 0;
     n = n < 1 ? 1 : n;
-    if (keep) seen[dev].store((unsigned long long)(smem + 1) << 16 | (unsigned)n, std::memory_order_release);
+    if (keep)
+      seen[dev][next[dev].fetch_add(1, std::memory_order_relaxed) % KEEP].store(
+          (unsigned long long)(smem + 1) << 16 | (unsigned)n, std::memory_order_release);
     return n;
   }
 };
