@@ -356,10 +356,17 @@ def range_(n1, n2, nprocs, irank):
     return a.value, b.value
 
 
+# torch's current stream as a handle, without a Stream object for it (a call
+# of torch's own generated code, not of its documented interface)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream=None):
     if stream is not None:
         return stream.cuda_stream
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 # ---------------------------------------------------------------- transforms
