@@ -403,9 +403,11 @@ int sph_timer_read(sph_plan* plan, double* ms, int* launches);
  * transforms (1, 2, 4, 8, dividing nlat/2, ring_pairs*nphi <= 8192);
  * z_cols: lm columns per CTA of the z transforms (a power of two <= 64,
  * z_cols*nz <= 4096; nz 16, 32, 48, 64, 96, 128, 192 and 256 keep their
- * fixed width, the one their two-step kernel is compiled for).  0 selects
- * the built-in choice.  Results do not
- * depend on the tile shapes beyond round-off.  Synchronises the device. */
+ * fixed width, the one their two-step kernel is compiled for).  Lengths
+ * without a compiled kernel take fewer ring pairs or columns where their
+ * buffers would not leave room for them in shared memory.  0 selects the
+ * built-in choice.  Results do not depend on the tile shapes beyond round-off.
+ * Synchronises the device. */
 int sph_plan_set_tiles(sph_plan* plan, int rows, int ring_pairs, int z_cols);
 
 /* Device status of a plan (no reference counterpart: the reference's
